@@ -298,7 +298,7 @@ typedef struct mc_render_params {
                                    TRAVERSAL_STACK_CAPACITY, PT:1038); 1..63 shrink the trace kernel's
                                    shared memory; a ray that needs more ends and the call returns
                                    MC_ERR_STACK_OVERFLOW (builds keep every 4-wide tree within 64) */
-    int32_t trace_threads;      /* trace block size: 256, or 128 (7 resident blocks per SM when the stack's
+    int32_t trace_threads;      /* trace block size: 256, or 128 (up to 8 resident blocks per SM when the stack's
                                    shared memory allows; launches without density grids, reference
                                    intersector; other launches keep 256). 0 with stack_entries 0: 128 with
                                    the stack the 4-wide trees can need (3 entries per level) when that is at
@@ -666,7 +666,7 @@ MC_API mc_status mc_rng_reset(mc_context* ctx, int32_t width, int32_t height, ui
  * waves of this render on this scene and BVH: the trace variant (persistent
  * or plain) and refill_threshold; the trace block shape (trace_threads 256,
  * or 128 with stack_entries cut to what the 4-wide tree can need, 3 per
- * level, when that lets 7 blocks share an SM); the queue capacity, as
+ * level, when that lets 7 or 8 blocks share an SM); the queue capacity, as
  * samples_per_wave (a wave's queues hold width x height x samples_per_wave
  * entries: the automatic choice, or twice it while spp and about 64M paths
  * allow; compared per sample); and use_graph. Cached per (device, layout,

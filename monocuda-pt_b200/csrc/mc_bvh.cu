@@ -990,15 +990,6 @@ __global__ void k_wide_fill(const float4* __restrict__ nodes, const int* __restr
     w[7] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-__global__ void k_reorder_prims(const float4* __restrict__ src, const int* __restrict__ rank, int n, float4* __restrict__ dst) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    int r = rank[k];
-    dst[(long long)r * 3 + 0] = src[(long long)k * 3 + 0];
-    dst[(long long)r * 3 + 1] = src[(long long)k * 3 + 1];
-    dst[(long long)r * 3 + 2] = src[(long long)k * 3 + 2];
-}
-
 __global__ void k_leaf_depth(const int32_t* __restrict__ parents, int N, int NI, int* depth) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= N) return;
@@ -1834,7 +1825,7 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
         return st != MC_OK ? st : status_from_device_flags(flags);
     }
     if (!palloc(ctx, &bvh->wide_nodes, (size_t)count * 128) ||
-        !palloc(ctx, &bvh->wide_prims, (size_t)N * 48)) {
+        !palloc(ctx, &bvh->records, (size_t)N * 64)) {
         cudaGetLastError();
         pool_free(ctx, rootOf);
         return set_error(MC_ERR_OOM, "mc_bvh_build: wide-node allocation failed");
@@ -1864,9 +1855,7 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
         h[28] = h[29] = h[30] = h[31] = 0.f;
         MC_CUDA(cudaMemcpyAsync(bvh->wide_nodes, h, sizeof(h), cudaMemcpyHostToDevice, ctx->stream));
     }
-    k_reorder_prims<<<grid_for(N, kBlock), kBlock, 0, ctx->stream>>>((const float4*)bvh->prims, rank, N,
-                                                                    (float4*)bvh->wide_prims);
-    MC_CUDA(cudaGetLastError());
+    if ((st = leaf_records(ctx, bvh->prims, rank, N, bvh->records)) != MC_OK) return st;
     MC_CUDA(cudaStreamSynchronize(ctx->stream));
     bvh->wide_count = count;
     bvh->layout = MC_BVH_LAYOUT_WIDE4;
@@ -2045,8 +2034,8 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
         }
         if (st == MC_ERR_UNSUPPORTED) {
             if (bvh->wide_nodes) pool_free(ctx, bvh->wide_nodes);
-            if (bvh->wide_prims) pool_free(ctx, bvh->wide_prims);
-            bvh->wide_nodes = bvh->wide_prims = nullptr;
+            if (bvh->records) pool_free(ctx, bvh->records);
+            bvh->wide_nodes = bvh->records = nullptr;
             if ((st = build_wide(ctx, bvh, dSeg, nseg, dWideRoot, coop)) != MC_OK) return fail(st);
             bvh->builder = MC_BVH_BUILDER_LBVH;
         }
@@ -2067,6 +2056,17 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
         bvh->wide_nodes = q;
         bvh->layout = MC_BVH_LAYOUT_WIDE4Q;
     }
+    if (bvh->layout == MC_BVH_LAYOUT_BINARY) {
+        if (!palloc(ctx, &bvh->records, (size_t)N * 64)) {
+            cudaGetLastError();
+            return fail(set_error(MC_ERR_OOM, "mc_bvh_build: leaf-record allocation failed"));
+        }
+        if ((st = leaf_records(ctx, bvh->prims, nullptr, N, bvh->records)) != MC_OK) return fail(st);
+        if (cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+            return fail(cuda_error(cudaGetLastError(), "mc_bvh_build (leaf records)", __FILE__, __LINE__));
+    }
+    pool_free(ctx, bvh->prims);  // the records replace the build's primitive stream
+    bvh->prims = nullptr;
     *out = bvh;
     return MC_OK;
 }
@@ -2150,7 +2150,7 @@ mc_status mc_bvh_free(mc_bvh* bvh) {
     if (prev != bvh->device) cudaSetDevice(bvh->device);
     // work on any stream may still read the tree (cudaFree would wait for the device too)
     cudaDeviceSynchronize();
-    void* bufs[] = {bvh->nodes, bvh->prims, bvh->wide_nodes, bvh->wide_prims, bvh->codes,
+    void* bufs[] = {bvh->nodes, bvh->prims, bvh->wide_nodes, bvh->records, bvh->codes,
                     bvh->ids, bvh->types, bvh->parents, bvh->ref_internal, bvh->ref_leaves};
     for (void* b : bufs) mc::pool_release(b);
     if (prev >= 0 && prev != bvh->device) cudaSetDevice(prev);
@@ -2203,7 +2203,8 @@ mc_status mc_bvh_export_traversal(const mc_bvh* bvh, void* d_nodes, void* d_prim
     if (d_nodes && nodeBytes > 0)
         MC_CUDA(cudaMemcpyAsync(d_nodes, wide ? bvh->wide_nodes : bvh->nodes, (size_t)nodeBytes, cudaMemcpyDeviceToDevice, s));
     if (d_prims && bvh->n > 0)
-        MC_CUDA(cudaMemcpyAsync(d_prims, wide ? bvh->wide_prims : bvh->prims, (size_t)bvh->n * 48, cudaMemcpyDeviceToDevice, s));
+        // the first 48 bytes of every record: the primitive and its identity
+        MC_CUDA(cudaMemcpy2DAsync(d_prims, 48, bvh->records, 64, 48, (size_t)bvh->n, cudaMemcpyDeviceToDevice, s));
     MC_CUDA(cudaStreamSynchronize(s));
     return MC_OK;
 }

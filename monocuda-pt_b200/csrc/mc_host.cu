@@ -249,7 +249,7 @@ mc_status mc_autotune(mc_context* ctx, const mc_bvh* bvh, const mc_scene_view* s
     cands.push_back({0, 8, 0, k, 256, 0});
     if ((st = tune(cands, &b)) == MC_OK) bestC = cands[b];
     // 2: 128-thread blocks with the stack the 4-wide tree needs (3 entries per
-    // level, rounded up to 8): 7 blocks per SM fit in shared memory up to 56
+    // level, rounded up to 8): 7 or 8 blocks per SM fit in shared memory up to 56
     // entries (persistent renders of wide layouts without density grids)
     const int need = bvh->wide_levels > 0 ? ((3 * bvh->wide_levels + 7) / 8) * 8 : 999;
     if (st == MC_OK && elapsed() < budget_ms && bestC.persistent && bvh->layout != MC_BVH_LAYOUT_BINARY && need <= 56 &&

@@ -145,11 +145,12 @@ struct mc_bvh {
     void* nodes = nullptr;             // traversal nodes (float4 records)
     long long node_count = 0;
     long long node_bytes = 0;
-    void* prims = nullptr;             // leaf-ordered primitive records, 48 B each
+    void* prims = nullptr;             // during the build: leaf-ordered primitives, 48 B each
+    void* records = nullptr;           // what the traversal reads: 64-byte primitive records (mc_traverse.cuh) in leaf
+                                       // order (binary layout) or in the reference's visit order (wide layouts)
     void* wide_nodes = nullptr;        // 4-wide nodes, 128 B each (layout MC_BVH_LAYOUT_WIDE4)
     long long wide_count = 0;
     int wide_levels = -1;              // levels of the greedy 4-wide tree (a ray's stack holds <= 3 per level), -1 unknown
-    void* wide_prims = nullptr;        // primitive records in reference visit (rank) order
     // reference representation (optional)
     uint32_t* codes = nullptr;
     int32_t* ids = nullptr;
@@ -217,6 +218,9 @@ mc_status render_items(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items
 mc_status check_params(const mc_render_params* p, const mc_scene_view* v);
 
 mc_status bvh_depth(mc_bvh* bvh);
+// The traversal's 64-byte records from n 48-byte primitives: record order[k]
+// (k when order is null) from primitive k (mc_render.cu).
+mc_status leaf_records(mc_context* ctx, const void* prims, const int* order, int n, void* records);
 mc_status context_counters(mc_context* ctx);
 // Guide kernels driven by device-side counts (guided renders).
 // Inputs of a queued path: its hit point and, per the guide's direction_input,

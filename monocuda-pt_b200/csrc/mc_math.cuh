@@ -17,6 +17,20 @@
 
 namespace mc {
 
+// Three-operand maximum and minimum: one instruction each on sm_100, where the
+// pipe of comparisons and selects, not the multiply-add pipe, is the traversal's
+// busiest. NaN operands are ignored, as fmaxf and fminf do.
+MC_D float max3(float a, float b, float c) {
+    float d;
+    asm("max.ftz.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+MC_D float min3(float a, float b, float c) {
+    float d;
+    asm("min.ftz.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
 // PT:105-158 vec3. Member-wise operators; normalize divides each component.
 struct V3 {
     float x, y, z;
@@ -105,28 +119,35 @@ MC_D bool hit_box(const RayInv& r, float lox, float loy, float loz, float hix, f
 
 // ---------------------------------------------------------------------------
 // Ray / triangle, PT:715-741 hit_triangle (plane + three edge signs; the
-// reference's test, not watertight).
+// reference's test, not watertight). The unit normal comes from the caller
+// (triangle_normal, computed once per triangle). limit: a plane farther than
+// it is no hit the caller would take, so the edges are not tested. The three
+// edge signs are combined without branches: lanes of a warp that leave early
+// would wait for the others anyway.
 // ---------------------------------------------------------------------------
-MC_D bool hit_triangle_ref(const V3& v0, const V3& v1, const V3& v2, const V3& o, const V3& d, float& tout) {
+MC_D V3 triangle_normal(const V3& v0, const V3& v1, const V3& v2) {
     V3 edge1 = v1 - v0;
     V3 edge2 = v2 - v0;
-    V3 nrm = edge1.cross(edge2).normalize();
+    return edge1.cross(edge2).normalize();
+}
+
+MC_D bool hit_triangle_ref(const V3& v0, const V3& v1, const V3& v2, const V3& nrm, const V3& o, const V3& d, float limit,
+                           float& tout) {
     float denom = d.dot(nrm);
-    if (fabsf(denom) < 1e-6f) return false;
     float t = (v0 - o).dot(nrm) / denom;
-    if (t < 0.0001f) return false;
+    if (fabsf(denom) < 1e-6f || t < 0.0001f || !(t <= limit)) return false;
     V3 p = o + d * t;
     V3 e0 = v1 - v0;
     V3 p0 = p - v0;
-    if (nrm.dot(e0.cross(p0)) < 0) return false;
+    const float s0 = nrm.dot(e0.cross(p0));
     V3 e1 = v2 - v1;
     V3 p1 = p - v1;
-    if (nrm.dot(e1.cross(p1)) < 0) return false;
+    const float s1 = nrm.dot(e1.cross(p1));
     V3 e2 = v0 - v2;
     V3 p2 = p - v2;
-    if (nrm.dot(e2.cross(p2)) < 0) return false;
+    const float s2 = nrm.dot(e2.cross(p2));
     tout = t;
-    return true;
+    return !(min3(s0, s1, s2) < 0.0f);
 }
 
 // Watertight ray/triangle test (Woop, Benthin, Wald, "Watertight Ray/Triangle
@@ -198,7 +219,10 @@ MC_D bool hit_sphere_ref(const V3& c0, const V3& c1, bool moving, float radius, 
                          float& tout, bool& frontFace, V3& outward) {
     V3 cc = sphere_center_at(c0, c1, moving, time);
     V3 oc = cc - o;
-    float tc = oc.dot(d) / d.dot(d);
+    // |d|^2 with its contraction written out: left to the compiler, which of
+    // the first two squares is rounded depends on the code around the call
+    float dd = __fmaf_rn(d.z, d.z, __fmaf_rn(d.x, d.x, __fmul_rn(d.y, d.y)));
+    float tc = oc.dot(d) / dd;
     V3 closest = o + d * tc;
     float dist2 = (cc - closest).length_squared();
     float disc = radius * radius - dist2;

@@ -158,13 +158,16 @@ MC_D void flush_counts(const TraceArgs& a, const TravCount& c) {
 }
 
 enum { RAY_EXTEND = 0, RAY_SHADOW_ANY = 1, RAY_SHADOW_MEDIUM = 2 };
+// A lane of the trace kernel: no ray, a ray in flight, or a ray whose
+// traversal ended and whose result is not written yet.
+enum { LANE_FREE = 0, LANE_RUNNING = 1, LANE_DONE = 2, LANE_OCCLUDED = 3 };
 
 // Finishes one ray. Returns true when the lane is free again. GRID: the
 // launch's scenes hold density grids (the crossing bookkeeping for
 // k_ratio_track is compiled in only then).
-template <int ISECT, bool GRID>
+template <int ISECT, bool GRID, class Stack>
 MC_D bool finish_ray(const TraceArgs& a, const TraceScene& ts, const mc_triangle_cold* cold, const mc_sphere* spheres,
-                     TravState& s, int step, int kind, int slot, float& T, float& travelled, int& crossings) {
+                     TravState& s, const Stack& stack, int step, int kind, int slot, float& T, float& travelled, int& crossings) {
     if (kind == RAY_EXTEND) {
         int type = -1, id = -1, did = 0;
         if (s.hitLeaf >= 0) {
@@ -206,13 +209,8 @@ MC_D bool finish_ray(const TraceArgs& a, const TraceScene& ts, const mc_triangle
         } else {
             bool front;
             if (type == 1) {
-                const float4* rec = ts.prims + (long long)s.hitLeaf * 3;
-                float4 r0 = __ldg(rec), r1 = __ldg(rec + 1), r2 = __ldg(rec + 2);
-                V3 v0(r0.x, r0.y, r0.z), v1(r0.w, r1.x, r1.y), v2(r1.z, r1.w, r2.x);
-                V3 e1 = v1 - v0;
-                V3 e2 = v2 - v0;
-                V3 nrm = e1.cross(e2).normalize();
-                front = s.r.d.dot(nrm) < 0.0f;
+                const float4 n4 = ldg4(leaf_record(ts, s.hitLeaf) + 3);
+                front = s.r.d.dot(V3(n4.x, n4.y, n4.z)) < 0.0f;
             } else {
                 const mc_sphere& sp = spheres[id];
                 float tt;
@@ -247,10 +245,7 @@ MC_D bool finish_ray(const TraceArgs& a, const TraceScene& ts, const mc_triangle
                 done = true;
             } else {
                 s.r.o = hp;
-                s.tmax = remaining;
-                s.hitLeaf = -1;
-                s.node = ts.root;
-                s.sp = 0;
+                trav_restart(s, stack, remaining, ts.root);
             }
         }
     }
@@ -280,15 +275,30 @@ MC_D bool finish_ray(const TraceArgs& a, const TraceScene& ts, const mc_triangle
 // BATCH: rays of several scenes share the launch; each lane reads its ray's
 // scene from the wave table. A single-scene launch reads the scene from the
 // kernel parameters instead, which costs no registers.
-// THREADS: 256 (3 resident blocks of up to 85 registers, the default) or 128
-// (7 resident blocks of up to 73 registers: 28 warps per SM instead of 24
-// when the traversal stack is short enough for 7 blocks' shared memory; a
-// variant the autotuner may pick for single-scene launches).
+// THREADS: 256 (3 resident blocks of up to 85 registers) or 128 (8 resident
+// blocks of 64 registers: 32 warps per SM instead of 24 when the traversal
+// stack is short enough for 8 blocks' shared memory; compiled for the reference
+// intersector without density grids, the default there).
+//
+// What bounds it: on incoherent rays the L1's data pipe (71 % of its peak on
+// the aperture room's bounces, the issue slots at 58 %, the pipe of compares
+// and selects at 43 %), on coherent ones issue; and at the end of a launch the
+// latency of its longest rays' steps. Hence: a node is three 32-byte loads and
+// one of 16 bytes (7 of 16 before) and a leaf two of 32 (3 of 16 plus the
+// normal's arithmetic), a wavefront of the data pipe each for a lane of its
+// own; planes of two children per add and multiply; a partial sort of the
+// children; results written by all finished lanes together at the refill. 1M
+// scattered rays on 500k triangles 2.28 -> 1.90 ms, the trace of a 1080p frame
+// of 3.9M triangles about 25 -> 22.5 ms, the 600x600 spheres frame 3.36 -> 2.80
+// ms. Not kept: prefetching the next node or the leaves (+25 % time on the
+// room: one more access per visit), near planes by address instead of by
+// select (7 loads), dropping popped nodes beyond the hit (4 % fewer visits,
+// 5 % more time for the wider stack entries).
 #ifndef MC_TRACE_MIN_BLOCKS
 #define MC_TRACE_MIN_BLOCKS 3
 #endif
 #ifndef MC_TRACE128_MIN_BLOCKS
-#define MC_TRACE128_MIN_BLOCKS 7
+#define MC_TRACE128_MIN_BLOCKS 8
 #endif
 constexpr int kTraceThreads = 256;
 template <int ISECT, int MED, bool COUNT, int LAY, bool BATCH, int THREADS = kTraceThreads>
@@ -301,13 +311,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? MC_TRACE_MIN_BLOCKS 
     const int extCount = a.extCount ? min(*a.extCount, a.queueCap) : a.extN;
     const int shCount = a.shCount ? min(*a.shCount, a.queueCap) : a.shN;
     const int total = extCount + shCount;
-#if MC_SMEM_STACK
     extern __shared__ int traceStack[];
-    const SharedStack<THREADS> stack{traceStack + threadIdx.x};
-#else
-    int stackMem[MC_STACK_CAPACITY];
-    const LocalStack stack{stackMem};
-#endif
+    const SharedStack<THREADS> stack(traceStack, a.stackCap);
     TravState s;
     TraceScene tsLane;
     tsLane.nodes = nullptr;
@@ -316,25 +321,49 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? MC_TRACE_MIN_BLOCKS 
     const TraceScene& ts = BATCH ? tsLane : a.ts0;
     WatertightRay w;
     w.kx = 0; w.ky = 1; w.kz = 2; w.sx = w.sy = w.sz = 0.f;
-    bool has = false, exhausted = total == 0;
+    bool exhausted = total == 0;
+    // lanes a warp fills: all 32, or fewer when the rays would not fill every
+    // warp of the grid otherwise. A lane then waits for fewer others' divergent
+    // steps, and such a launch is as long as its longest ray: 5,003 occlusion
+    // rays 122 -> 95 us, 16 small scenes built and rendered 2.71 -> 2.55 ms
+    const int warps = gridDim.x * (THREADS / 32);
+    const int width = a.oneShot ? 32 : min(32, (total + warps - 1) / warps);
+    const int floor = width - min(width, a.refill);  // running lanes at or below which the warp refills
+    int state = LANE_FREE;
     int kind = 0, slot = 0, crossings = 0, sid = 0;
     float T = 1.f, travelled = 0.f;
     while (true) {
-        if (!exhausted) {
-            unsigned idle = __ballot_sync(kFull, !has);
-            int cnt = __popc(idle);
-            if (cnt >= a.refill) {
-                int leader = __ffs(idle) - 1;
+        const unsigned running = __ballot_sync(kFull, state == LANE_RUNNING);
+        // finished rays wait until enough lanes are idle, then one pass writes
+        // all their results and the freed lanes take new rays
+        if (exhausted ? running != kFull : __popc(running) <= floor) {
+            if (state > LANE_RUNNING) {
+                const mc_triangle_cold* cold = a.cold0;
+                const mc_sphere* spheres = a.spheres0;
+                if (BATCH && MED != 0 && kind == RAY_SHADOW_MEDIUM) {
+                    cold = a.tab->scenes[sid].cold;
+                    spheres = a.tab->scenes[sid].spheres;
+                }
+                const int step = state == LANE_OCCLUDED ? STEP_OCCLUDED : STEP_DONE;
+                state = finish_ray<ISECT, MED == 2>(a, ts, cold, spheres, s, stack, step, kind, slot, T, travelled, crossings)
+                            ? LANE_FREE
+                            : LANE_RUNNING;
+            }
+            if (!exhausted) {
+                const unsigned idle = __ballot_sync(kFull, state == LANE_FREE);
+                const int take = width - (32 - __popc(idle));
                 int base = 0;
                 if (a.oneShot) {
                     // plain wavefront (PT:3376-3397): one ray per thread, no refill
                     base = blockIdx.x * blockDim.x + (threadIdx.x & ~31);
                 } else {
-                    if (lane == leader) base = atomicAdd(a.work, cnt);
-                    base = __shfl_sync(kFull, base, leader);
+                    const int leader = __ffs(idle) - 1;
+                    if (lane == leader) base = atomicAdd(a.work, take);
+                    base = __shfl_sync(kFull, base, max(leader, 0));
                 }
-                if (!has) {
-                    int q = base + __popc(idle & ltmask);
+                const int nth = __popc(idle & ltmask);
+                if (state == LANE_FREE && nth < take) {
+                    int q = base + nth;
                     if (q < total) {
                         V3 o, d;
                         float time, tmax;
@@ -366,38 +395,21 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? MC_TRACE_MIN_BLOCKS 
                             tsLane.prims = S->prims;
                             tsLane.root = S->root;
                         }
-                        has = true;
-                        if (kind == RAY_SHADOW_MEDIUM && tmax <= 0.0f) {
-                            // PT:2880-2881: nothing left to traverse, transmittance 1
-                            // (no leaf, so the material arrays are not read)
-                            s.tmax = tmax;
-                            s.hitLeaf = -1;
-                            finish_ray<ISECT, MED == 2>(a, ts, nullptr, nullptr, s, STEP_DONE, kind, slot, T, travelled, crossings);
-                            has = false;
-                        }
-                        if (has) {
-                            trav_begin(s, o, d, time, tmax, ts.root);
-                            if (ISECT == MC_ISECT_WATERTIGHT) w = make_watertight(d);
-                        }
+                        trav_begin(s, stack, o, d, time, tmax, ts.root);
+                        if (ISECT == MC_ISECT_WATERTIGHT) w = make_watertight(d);
+                        // PT:2880-2881: a medium segment with nothing left to
+                        // traverse ends here (no leaf: transmittance 1)
+                        state = kind == RAY_SHADOW_MEDIUM && tmax <= 0.0f ? LANE_DONE : LANE_RUNNING;
                     }
                 }
-                if (a.oneShot || base + cnt >= total) exhausted = true;
+                if (a.oneShot || base + take >= total) exhausted = true;
             }
+            if (exhausted && __ballot_sync(kFull, state != LANE_FREE) == 0u) break;
         }
-        if (exhausted && __ballot_sync(kFull, has) == 0u) break;
-        if (has) {
-            int r = (kind == RAY_SHADOW_ANY)
-                        ? trav_step_layout<true, ISECT, COUNT, LAY>(ts, s, stack, w, a.err, &cnt, a.stackCap)
-                        : trav_step_layout<false, ISECT, COUNT, LAY>(ts, s, stack, w, a.err, &cnt, a.stackCap);
-            if (r != STEP_CONTINUE) {
-                const mc_triangle_cold* cold = a.cold0;
-                const mc_sphere* spheres = a.spheres0;
-                if (BATCH && MED != 0 && kind == RAY_SHADOW_MEDIUM) {
-                    cold = a.tab->scenes[sid].cold;
-                    spheres = a.tab->scenes[sid].spheres;
-                }
-                if (finish_ray<ISECT, MED == 2>(a, ts, cold, spheres, s, r, kind, slot, T, travelled, crossings)) has = false;
-            }
+        if (state == LANE_RUNNING) {
+            const int r = (kind == RAY_SHADOW_ANY) ? trav_step_layout<true, ISECT, COUNT, LAY>(ts, s, stack, w, a.err, &cnt)
+                                                   : trav_step_layout<false, ISECT, COUNT, LAY>(ts, s, stack, w, a.err, &cnt);
+            if (r != STEP_CONTINUE) state = r == STEP_OCCLUDED ? LANE_OCCLUDED : LANE_DONE;
         }
     }
     if (COUNT) flush_counts(a, cnt);
@@ -1240,6 +1252,22 @@ __global__ void k_init_xorwow(curandState* states, int pixels, unsigned long lon
     if (p < pixels) curand_init(seed, p, 0, &states[p]);  // PT:2870
 }
 
+// A primitive's traversal record: its 48 bytes and, for a triangle, its unit
+// normal, computed here as hit_triangle_ref's callers used to per test.
+__global__ void k_leaf_records(const float4* __restrict__ prims, const int* __restrict__ order, int n,
+                               float4* __restrict__ records) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const float4 a = prims[(size_t)k * 3], b = prims[(size_t)k * 3 + 1], c = prims[(size_t)k * 3 + 2];
+    float4* r = records + (size_t)(order ? order[k] : k) * 4;
+    V3 nrm;
+    if (__float_as_int(c.z) == 1) nrm = triangle_normal(V3(a.x, a.y, a.z), V3(a.w, b.x, b.y), V3(b.z, b.w, c.x));
+    r[0] = a;
+    r[1] = b;
+    r[2] = c;
+    r[3] = make_float4(nrm.x, nrm.y, nrm.z, 0.f);
+}
+
 int occupancy_blocks(const void* fn, int sms, size_t smem = 0, int threads = 256) {
     int per = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, smem);
@@ -1286,7 +1314,7 @@ void launch_trace(mc_context* ctx, cudaStream_t stream, const TraceArgs& t0, int
     const bool small = t.threads == 128 && !count && isect == 0 && medium < 2;
     const int threads = small ? 128 : kTraceThreads;
     // the shared-memory stack holds stackCap entries per lane
-    const int smem = MC_SMEM_STACK ? threads * t.stackCap * (int)sizeof(int) : 0;
+    const int smem = threads * t.stackCap * (int)sizeof(int);
     TraceKernel fn = small ? trace_kernel_128(batch, layout, medium) : trace_kernel(batch, layout, count, medium, isect);
     const int key = medium + 3 * (isect ? 1 : 0) + 6 * (count ? 1 : 0) + 12 * (batch ? 1 : 0) + 24 * layout +
                     72 * (small ? 1 : 0);  // < 144
@@ -1311,6 +1339,12 @@ void launch_trace(mc_context* ctx, cudaStream_t stream, const TraceArgs& t0, int
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
+mc_status leaf_records(mc_context* ctx, const void* prims, const int* order, int n, void* records) {
+    k_leaf_records<<<(n + 255) / 256, 256, 0, ctx->stream>>>((const float4*)prims, order, n, (float4*)records);
+    MC_CUDA(cudaGetLastError());
+    return MC_OK;
+}
+
 mc_status ensure_wave(mc_context* ctx, int capacity) {
     WaveBuffers& w = ctx->wave;
     if (w.capacity >= capacity && w.block.ptr) return MC_OK;
@@ -1404,7 +1438,7 @@ static SceneGPU scene_gpu(mc_context* ctx, const mc_bvh* shared, const WaveItem&
     const mc_bvh* bvh = it.bvh ? it.bvh : shared;
     const bool wide = bvh->layout != MC_BVH_LAYOUT_BINARY;
     g.nodes = (const float4*)(wide ? bvh->wide_nodes : bvh->nodes);
-    g.prims = (const float4*)(wide ? bvh->wide_prims : bvh->prims);
+    g.prims = (const float4*)bvh->records;
     g.root = it.root;
     g.spheres = it.view->spheres;
     g.hot = it.view->tri_hot;
@@ -1434,11 +1468,25 @@ static SceneGPU scene_gpu(mc_context* ctx, const mc_bvh* shared, const WaveItem&
 static void set_single_scene(TraceArgs& t, const mc_bvh* bvh, int root, const mc_scene_view* v) {
     const bool wide = bvh->layout != MC_BVH_LAYOUT_BINARY;
     t.ts0.nodes = (const float4*)(wide ? bvh->wide_nodes : bvh->nodes);
-    t.ts0.prims = (const float4*)(wide ? bvh->wide_prims : bvh->prims);
+    t.ts0.prims = (const float4*)bvh->records;
     t.ts0.root = root;
     t.medium0 = v->has_medium;
     t.cold0 = v->tri_cold;
     t.spheres0 = v->spheres;
+}
+
+// Levels of a greedy 4-wide tree, -1 for other trees.
+static int shape_levels(const mc_bvh* b) { return b->layout == MC_BVH_LAYOUT_BINARY || b->wide_levels <= 0 ? -1 : b->wide_levels; }
+
+// The default launch shape: 128 threads when every tree of the launch is a
+// greedy 4-wide collapse whose stack need (3 entries per level, rounded up to
+// 8) lets 7 or 8 blocks share an SM; results do not depend on it.
+static void default_shape(TraceArgs& t, int levels, int isect) {
+    const int need = levels > 0 ? ((3 * levels + 7) / 8) * 8 : 999;
+    if (need <= 56 && isect == MC_ISECT_REFERENCE) {
+        t.threads = 128;
+        t.stackCap = need;
+    }
 }
 
 // Runs waves until every item has rendered its spp samples. All items share
@@ -1533,20 +1581,12 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
     ta.stackCap = p0.stack_entries;
     ta.threads = p0.trace_threads;
     if (ta.threads == 0 && ta.stackCap == 0) {
-        // by default the 128-thread shape (7 blocks per SM) when every tree of
-        // the wave is a greedy 4-wide collapse whose stack need (3 entries per
-        // level, rounded up to 8) lets 7 blocks share an SM; the image does
-        // not depend on it
         int levels = 0;
         for (int i = 0; i < n && levels >= 0; i++) {
-            const mc_bvh* b = items[i].bvh ? items[i].bvh : bvh;
-            levels = (b->layout == MC_BVH_LAYOUT_BINARY || b->wide_levels <= 0) ? -1 : std::max(levels, b->wide_levels);
+            const int l = shape_levels(items[i].bvh ? items[i].bvh : bvh);
+            levels = l < 0 ? -1 : std::max(levels, l);
         }
-        const int need = levels > 0 ? ((3 * levels + 7) / 8) * 8 : 999;
-        if (need <= 56 && isect == MC_ISECT_REFERENCE) {
-            ta.threads = 128;
-            ta.stackCap = need;
-        }
+        default_shape(ta, levels, isect);
     }
     ta.refill = (p0.refill_threshold > 0 && p0.refill_threshold <= 32) ? p0.refill_threshold : 8;  // PT:3400
     if (countVisits) ta.counts = (unsigned long long*)(ctx->d_stats + 2 * MC_MAX_DEPTH_STATS);
@@ -1952,8 +1992,9 @@ mc_status render_items(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items
     return finish_stats(ctx, tm, paths, stats);
 }
 
-// The single-scene trace arguments of the ray-set entry points.
-static void ray_set_scene(TraceArgs& t, const mc_bvh* bvh, const mc_scene_view* scene) {
+// The single-scene trace arguments and launch shape of the ray-set entry points.
+static void ray_set_scene(TraceArgs& t, const mc_bvh* bvh, const mc_scene_view* scene, int isect) {
+    default_shape(t, shape_levels(bvh), isect);
     set_single_scene(t, bvh, bvh->layout != MC_BVH_LAYOUT_BINARY ? bvh->wide_roots[0] : bvh->bin_roots[0], scene);
 }
 
@@ -2091,7 +2132,7 @@ mc_status mc_trace_closest(mc_context* ctx, const mc_bvh* bvh, const mc_scene_vi
     MC_CUDA(cudaMemsetAsync(ctx->d_error, 0, sizeof(int), ctx->stream));
     mc::TraceArgs t;
     std::memset(&t, 0, sizeof(t));
-    mc::ray_set_scene(t, bvh, scene);
+    mc::ray_set_scene(t, bvh, scene, intersector);
     t.err = ctx->d_error;
     t.refill = 8;
     size_t N = (size_t)n;
@@ -2123,7 +2164,7 @@ mc_status mc_trace_any(mc_context* ctx, const mc_bvh* bvh, const mc_scene_view* 
     MC_CUDA(cudaMemsetAsync(ctx->d_error, 0, sizeof(int), ctx->stream));
     mc::TraceArgs t;
     std::memset(&t, 0, sizeof(t));
-    mc::ray_set_scene(t, bvh, scene);
+    mc::ray_set_scene(t, bvh, scene, intersector);
     t.err = ctx->d_error;
     t.refill = 8;
     size_t N = (size_t)n;

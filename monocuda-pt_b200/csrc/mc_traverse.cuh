@@ -3,8 +3,8 @@
 // Binary layout: one 64-byte record per internal node holding BOTH children's
 // boxes and references (leaf child k -> ~k), so a traversal step is one
 // contiguous 64-byte read instead of the reference's node read plus two child
-// box reads (PT:1276-1321). Leaves are 48-byte primitive records in leaf
-// (sorted Morton) order: a triangle's three vertices plus its id and type.
+// box reads (PT:1276-1321). Leaves are 64-byte primitive records in leaf
+// (sorted Morton) order: a triangle's three vertices, id, type and unit normal.
 //
 // The visit order and every test follow the reference's stepTraversal /
 // traverseAnyHit (PT:1152-1321): both child boxes are tested against the
@@ -14,44 +14,30 @@
 #pragma once
 #include "mc_math.cuh"
 
-// Leaf children of a 4-wide node: one loop over the lane's hit leaves (1) or
-// one predicated block per child slot (0).
-#ifndef MC_LEAF_LOOP
-#define MC_LEAF_LOOP 1
-#endif
-// Traversal stack of the trace kernel: shared memory (1; 64 KB per 256-thread
-// block, measured 2 % faster on B200) or local memory (0).
-#ifndef MC_SMEM_STACK
-#define MC_SMEM_STACK 1
-#endif
-// 4-wide steps: start fetching the next node (the nearest hit internal child,
-// else the top of the stack) into L1 before the leaf children are intersected,
-// so its latency overlaps theirs (1), or not (0).
-#ifndef MC_PREFETCH_NEXT
-#define MC_PREFETCH_NEXT 0
-#endif
-
 namespace mc {
 
 enum { STEP_CONTINUE = 0, STEP_DONE = 1, STEP_OCCLUDED = 2 };
 
 struct TraceScene {
     const float4* __restrict__ nodes;   // binary: 4 float4 per internal node; wide: 8
-    const float4* __restrict__ prims;   // 3 float4 per leaf
+    const float4* __restrict__ prims;   // primitive records, 4 float4 per leaf
     int root;                           // root node of this scene (batched builds share the arrays)
 };
 
-// A lane's traversal stack in local memory.
-struct LocalStack {
-    int* p;
-    MC_D int& operator[](int i) const { return p[i]; }
-};
-// A lane's traversal stack in shared memory: entry i of the block's thread t at
-// base[i * STRIDE + t], so a warp's accesses fall in 32 distinct banks at any depths.
+// A lane's traversal stack in shared memory: entry i of the block's thread t
+// at word i * STRIDE + t, so a warp's accesses fall in 32 distinct banks at
+// any depths. Positions are byte offsets from the block's array, so a push or
+// a pop is one access and one addition.
 template <int STRIDE>
 struct SharedStack {
-    int* p;  // base + threadIdx.x
-    MC_D int& operator[](int i) const { return p[i * STRIDE]; }
+    char* base;   // the block's array
+    int bottom;   // this lane's entry 0
+    int limit;    // one past this lane's last entry
+    MC_D SharedStack(int* array, int cap)
+        : base(reinterpret_cast<char*>(array)), bottom((int)threadIdx.x * 4), limit((int)threadIdx.x * 4 + cap * STRIDE * 4) {}
+    static constexpr int kStep = STRIDE * 4;
+    MC_D void put(int at, int v) const { *reinterpret_cast<int*>(base + at) = v; }
+    MC_D int get(int at) const { return *reinterpret_cast<const int*>(base + at); }
 };
 
 // Traversal state of one ray in one lane.
@@ -61,30 +47,49 @@ struct TravState {
     float tmax;     // closest distance so far (closest) or the segment length (any hit)
     int hitLeaf;    // leaf slot of the closest hit, -1 none
     int node;
-    int sp;
+    int sp;         // stack position (SharedStack byte offset)
 };
 
-MC_D void trav_begin(TravState& s, const V3& o, const V3& d, float time, float tmax, int root) {
-    s.r = make_ray_inv(o, d);
-    s.time = time;
+template <class Stack>
+MC_D void trav_restart(TravState& s, const Stack& stack, float tmax, int root) {
     s.tmax = tmax;
     s.hitLeaf = -1;
     s.node = root;
-    s.sp = 0;
+    s.sp = stack.bottom;
+}
+
+template <class Stack>
+MC_D void trav_begin(TravState& s, const Stack& stack, const V3& o, const V3& d, float time, float tmax, int root) {
+    s.r = make_ray_inv(o, d);
+    s.time = time;
+    trav_restart(s, stack, tmax, root);
 }
 
 MC_D float4 ldg4(const float4* p) { return __ldg(p); }
+// 32 bytes (32-byte aligned) as one load.
+MC_D void ldg8(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
+// A leaf's 64-byte record (two sectors of one line): a triangle's three
+// vertices, its id and type, and its unit normal; a sphere's centers, radius
+// and motion flag in the vertices' place.
+MC_D const float4* leaf_record(const TraceScene& sc, int k) { return sc.prims + (size_t)((unsigned)k * 4u); }
 
 // Intersects leaf slot k; returns true and t when the primitive is hit with
 // t in the reference's accepted range (hit_* internal checks).
 template <int ISECT>
 MC_D bool leaf_hit(const TraceScene& sc, int k, const TravState& s, const WatertightRay& w, float& t) {
-    const float4* rec = sc.prims + (long long)k * 3;
-    float4 a = ldg4(rec + 0), b = ldg4(rec + 1), c = ldg4(rec + 2);
+    const float4* rec = leaf_record(sc, k);
+    float4 a, b, c, n;
+    ldg8(rec, a, b);
+    ldg8(rec + 2, c, n);
     int type = __float_as_int(c.z);
     if (type == 1) {
         V3 v0(a.x, a.y, a.z), v1(a.w, b.x, b.y), v2(b.z, b.w, c.x);
-        if (ISECT == 0) return hit_triangle_ref(v0, v1, v2, s.r.o, s.r.d, t);
+        if (ISECT == 0) return hit_triangle_ref(v0, v1, v2, V3(n.x, n.y, n.z), s.r.o, s.r.d, s.tmax, t);
         return hit_triangle_watertight(w, v0, v1, v2, s.r.o, t);
     }
     bool front;
@@ -101,11 +106,10 @@ struct TravCount {
     int leaves = 0;
 };
 
-// cap: stack entries available to the lane (at most MC_STACK_CAPACITY); a push
-// beyond it ends the ray and sets MC_DEVERR_STACK.
-template <bool ANY, int ISECT, bool COUNT = false, class Stack = LocalStack>
+// A push beyond the lane's stack ends the ray and sets MC_DEVERR_STACK.
+template <bool ANY, int ISECT, bool COUNT, class Stack>
 MC_D int trav_step(const TraceScene& sc, TravState& s, const Stack& stack, const WatertightRay& w, int* err,
-                   TravCount* cnt, int cap) {
+                   TravCount* cnt) {
     const float4* nd = sc.nodes + (long long)s.node * 4;
     float4 a = ldg4(nd + 0), b = ldg4(nd + 1), c = ldg4(nd + 2), d = ldg4(nd + 3);
     int lref = __float_as_int(d.x), rref = __float_as_int(d.y);
@@ -140,17 +144,17 @@ MC_D int trav_step(const TraceScene& sc, TravState& s, const Stack& stack, const
     }
     bool tL = oL && !lLeaf, tR = oR && !rLeaf;
     if (!tL && !tR) {
-        if (s.sp == 0) return STEP_DONE;
-        s.sp--;
-        s.node = stack[s.sp];
+        if (s.sp == stack.bottom) return STEP_DONE;
+        s.sp -= Stack::kStep;
+        s.node = stack.get(s.sp);
     } else {
         if (tL && tR) {
-            if (s.sp >= cap) {
+            if (s.sp >= stack.limit) {
                 atomicOr(err, MC_DEVERR_STACK);
                 return STEP_DONE;
             }
-            stack[s.sp] = rref;
-            s.sp++;
+            stack.put(s.sp, rref);
+            s.sp += Stack::kStep;
         }
         s.node = tL ? lref : rref;
     }
@@ -167,18 +171,32 @@ MC_D int trav_step(const TraceScene& sc, TravState& s, const Stack& stack, const
 // tested with the reference's slab arithmetic (no per-axis early exit is needed:
 // the three-axis test returns the same boolean).
 // ---------------------------------------------------------------------------
-MC_D void slab4(const RayInv& r, float lx, float ly, float lz, float hx, float hy, float hz, float tfar, float& tnear,
-                bool& hit) {
-    float e0 = (lx - r.o.x) * r.ix, x0 = (hx - r.o.x) * r.ix;
-    if (r.ix < 0.0f) { float t = e0; e0 = x0; x0 = t; }
-    float e1 = (ly - r.o.y) * r.iy, x1 = (hy - r.o.y) * r.iy;
-    if (r.iy < 0.0f) { float t = e1; e1 = x1; x1 = t; }
-    float e2 = (lz - r.o.z) * r.iz, x2 = (hz - r.o.z) * r.iz;
-    if (r.iz < 0.0f) { float t = e2; e2 = x2; x2 = t; }
-    float n = fmaxf(fmaxf(fmaxf(0.0001f, e0), e1), e2);
-    float f = fminf(fminf(fminf(tfar, x0), x1), x2);
-    hit = !(f <= n);
-    tnear = n;
+// (plane - o) * (1 / d) of the four children's planes on one axis, two values
+// per instruction (the same roundings as four subtractions and four
+// multiplications).
+MC_D float2 slab_t2(float u, float v, float o, float i) {
+    float2 r;
+    asm("{\n\t.reg .b64 a, b, c;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmov.b64 c, {%5, %5};\n\t"
+        "add.rn.ftz.f32x2 a, a, b;\n\tmul.rn.ftz.f32x2 a, a, c;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(u), "f"(v), "f"(-o), "f"(i));
+    return r;
+}
+MC_D float4 slab_t4(const float4& p, float o, float i) {
+    const float2 a = slab_t2(p.x, p.y, o, i), b = slab_t2(p.z, p.w, o, i);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// The reference's slab test from a box's entry (e) and exit (x) distances per
+// axis, already swapped by the sign of the direction.
+MC_D bool slab_hit(float e0, float e1, float e2, float x0, float x1, float x2, float tfar, float& tnear) {
+    tnear = fmaxf(max3(0.0001f, e0, e1), e2);
+    return !(fminf(min3(tfar, x0, x1), x2) <= tnear);
+}
+
+MC_D float4 pick(bool c, const float4& a, const float4& b) {
+    return make_float4(c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z, c ? a.w : b.w);
 }
 
 MC_D void cswap(float& ka, int& va, float& kb, int& vb) {
@@ -202,14 +220,15 @@ MC_D float q_scale(unsigned exps, int axis) {
 
 // QUANT: 64-byte quantised nodes with conservative boxes (more boxes pass; the
 // leaf tests and the rank rule decide the hit as with exact boxes).
-template <bool ANY, int ISECT, bool COUNT = false, class Stack = LocalStack, bool QUANT = false>
+template <bool ANY, int ISECT, bool COUNT, class Stack, bool QUANT>
 MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, const WatertightRay& w, int* err,
-                    TravCount* cnt, int cap) {
-    float4 lx, ly, lz, hx, hy, hz, rf;
+                    TravCount* cnt) {
+    float4 lx, ly, lz, hx, hy, hz, rf;  // low and high planes of the four children, their references
     if (QUANT) {
-        const float4* nd = sc.nodes + (long long)s.node * 4;
-        const float4 h = ldg4(nd + 0), q0 = ldg4(nd + 1), q1 = ldg4(nd + 2);
-        rf = ldg4(nd + 3);
+        const float4* nd = sc.nodes + (size_t)((unsigned)s.node * 4u);
+        float4 h, q0, q1;
+        ldg8(nd, h, q0);
+        ldg8(nd + 2, q1, rf);
         const unsigned ex = (unsigned)__float_as_int(h.w);
         const float sx = q_scale(ex, 0), sy = q_scale(ex, 1), sz = q_scale(ex, 2);
         lx = q_planes(h.x, sx, (unsigned)__float_as_int(q0.x));
@@ -219,44 +238,60 @@ MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, cons
         hy = q_planes(h.y, sy, (unsigned)__float_as_int(q1.x));
         hz = q_planes(h.z, sz, (unsigned)__float_as_int(q1.y));
     } else {
-        const float4* nd = sc.nodes + (long long)s.node * 8;
-        lx = ldg4(nd + 0); ly = ldg4(nd + 1); lz = ldg4(nd + 2);
-        hx = ldg4(nd + 3); hy = ldg4(nd + 4); hz = ldg4(nd + 5);
+        const float4* nd = sc.nodes + (size_t)((unsigned)s.node * 8u);
+        ldg8(nd, lx, ly);
+        ldg8(nd + 2, lz, hx);
+        ldg8(nd + 4, hy, hz);
         rf = ldg4(nd + 6);
     }
-    int ref[4] = {__float_as_int(rf.x), __float_as_int(rf.y), __float_as_int(rf.z), __float_as_int(rf.w)};
+    const bool sx = s.r.ix < 0.0f, sy = s.r.iy < 0.0f, sz = s.r.iz < 0.0f;
+    const float4 ax = slab_t4(pick(sx, hx, lx), s.r.o.x, s.r.ix), bx = slab_t4(pick(sx, lx, hx), s.r.o.x, s.r.ix);
+    const float4 ay = slab_t4(pick(sy, hy, ly), s.r.o.y, s.r.iy), by = slab_t4(pick(sy, ly, hy), s.r.o.y, s.r.iy);
+    const float4 az = slab_t4(pick(sz, hz, lz), s.r.o.z, s.r.iz), bz = slab_t4(pick(sz, lz, hz), s.r.o.z, s.r.iz);
+    const int ref[4] = {__float_as_int(rf.x), __float_as_int(rf.y), __float_as_int(rf.z), __float_as_int(rf.w)};
     float tn[4];
     bool hit[4];
-    slab4(s.r, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x, s.tmax, tn[0], hit[0]);
-    slab4(s.r, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y, s.tmax, tn[1], hit[1]);
-    slab4(s.r, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z, s.tmax, tn[2], hit[2]);
-    slab4(s.r, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w, s.tmax, tn[3], hit[3]);
+    hit[0] = slab_hit(ax.x, ay.x, az.x, bx.x, by.x, bz.x, s.tmax, tn[0]);
+    hit[1] = slab_hit(ax.y, ay.y, az.y, bx.y, by.y, bz.y, s.tmax, tn[1]);
+    hit[2] = slab_hit(ax.z, ay.z, az.z, bx.z, by.z, bz.z, s.tmax, tn[2]);
+    hit[3] = slab_hit(ax.w, ay.w, az.w, bx.w, by.w, bz.w, s.tmax, tn[3]);
     if (COUNT) cnt->visits++;
-#if MC_PREFETCH_NEXT
-    {
-        // the next node does not depend on the leaf tests below: the hit flags
-        // are taken against the distance before them, as in the choice further down
-        float kn = INFINITY;
-        int vn = -1;
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-            if (hit[c] && ref[c] >= 0 && ref[c] != MC_WIDE_EMPTY && tn[c] < kn) {
-                kn = tn[c];
-                vn = ref[c];
-            }
-        if (vn < 0 && s.sp > 0) vn = stack[s.sp - 1];
-        if (vn >= 0) {
-            const float4* nn = sc.nodes + (long long)vn * (QUANT ? 4 : 8);
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(nn));
-        }
-    }
-#endif
-    // leaf children first
-#if MC_LEAF_LOOP
-    // one loop over this lane's hit leaf children: a warp runs as many
-    // iterations as its busiest lane, not one predicated block per child slot
     unsigned lm = (hit[0] && ref[0] < 0 ? 1u : 0u) | (hit[1] && ref[1] < 0 ? 2u : 0u) |
                   (hit[2] && ref[2] < 0 ? 4u : 0u) | (hit[3] && ref[3] < 0 ? 8u : 0u);
+    // internal children, the nearest first; misses, leaves and empty slots
+    // (MC_WIDE_EMPTY, the largest int) as +inf
+    constexpr unsigned kLeafOrEmpty = (unsigned)MC_WIDE_EMPTY;
+    float k0 = (hit[0] && (unsigned)ref[0] < kLeafOrEmpty) ? tn[0] : INFINITY;
+    float k1 = (hit[1] && (unsigned)ref[1] < kLeafOrEmpty) ? tn[1] : INFINITY;
+    float k2 = (hit[2] && (unsigned)ref[2] < kLeafOrEmpty) ? tn[2] : INFINITY;
+    float k3 = (hit[3] && (unsigned)ref[3] < kLeafOrEmpty) ? tn[3] : INFINITY;
+    int v0 = ref[0], v1 = ref[1], v2 = ref[2], v3 = ref[3];
+    cswap(k0, v0, k1, v1);
+    cswap(k2, v2, k3, v3);
+    cswap(k0, v0, k2, v2);
+    int step = STEP_CONTINUE;
+    if (k0 == INFINITY) {
+        if (s.sp == stack.bottom) step = STEP_DONE;
+        else {
+            s.sp -= Stack::kStep;
+            s.node = stack.get(s.sp);
+        }
+    } else {
+        // push the others, continue with the nearest
+        const int extra = (k1 != INFINITY) + (k2 != INFINITY) + (k3 != INFINITY);
+        if (s.sp + extra * Stack::kStep > stack.limit) {
+            atomicOr(err, MC_DEVERR_STACK);
+            step = STEP_DONE;
+        } else {
+            if (k3 != INFINITY) { stack.put(s.sp, v3); s.sp += Stack::kStep; }
+            if (k1 != INFINITY) { stack.put(s.sp, v1); s.sp += Stack::kStep; }
+            if (k2 != INFINITY) { stack.put(s.sp, v2); s.sp += Stack::kStep; }
+            s.node = v0;
+        }
+    }
+    // the leaf children: one loop over this lane's hit leaf children (a warp
+    // runs as many iterations as its busiest lane, not one predicated block per
+    // child slot)
     while (lm) {
         const int c = __ffs(lm) - 1;
         lm &= lm - 1;
@@ -272,66 +307,21 @@ MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, cons
             }
         }
     }
-#else
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        if (hit[c] && ref[c] < 0) {
-            int k = ~ref[c];
-            float t;
-            if (COUNT) cnt->leaves++;
-            if (leaf_hit<ISECT>(sc, k, s, w, t)) {
-                if (ANY) {
-                    if (t > 0.0001f && t < s.tmax) return STEP_OCCLUDED;
-                } else if (t > 0.0001f && (t < s.tmax || (t == s.tmax && s.hitLeaf >= 0 && k < s.hitLeaf))) {
-                    s.tmax = t;
-                    s.hitLeaf = k;
-                }
-            }
-        }
-    }
-#endif
-    // internal children, nearest first: sort (tnear, ref) ascending, misses as +inf
-    float k0 = (hit[0] && ref[0] >= 0 && ref[0] != MC_WIDE_EMPTY) ? tn[0] : INFINITY;
-    float k1 = (hit[1] && ref[1] >= 0 && ref[1] != MC_WIDE_EMPTY) ? tn[1] : INFINITY;
-    float k2 = (hit[2] && ref[2] >= 0 && ref[2] != MC_WIDE_EMPTY) ? tn[2] : INFINITY;
-    float k3 = (hit[3] && ref[3] >= 0 && ref[3] != MC_WIDE_EMPTY) ? tn[3] : INFINITY;
-    int v0 = ref[0], v1 = ref[1], v2 = ref[2], v3 = ref[3];
-    cswap(k0, v0, k1, v1);
-    cswap(k2, v2, k3, v3);
-    cswap(k0, v0, k2, v2);
-    cswap(k1, v1, k3, v3);
-    cswap(k1, v1, k2, v2);
-    if (k0 == INFINITY) {
-        if (s.sp == 0) return STEP_DONE;
-        s.sp--;
-        s.node = stack[s.sp];
-        return STEP_CONTINUE;
-    }
-    // push the farther ones (farthest first), continue with the nearest
-    int extra = (k1 != INFINITY) + (k2 != INFINITY) + (k3 != INFINITY);
-    if (s.sp + extra > cap) {
-        atomicOr(err, MC_DEVERR_STACK);
-        return STEP_DONE;
-    }
-    if (k3 != INFINITY) stack[s.sp++] = v3;
-    if (k2 != INFINITY) stack[s.sp++] = v2;
-    if (k1 != INFINITY) stack[s.sp++] = v1;
-    s.node = v0;
-    return STEP_CONTINUE;
+    return step;
 }
 
 // LAY: MC_BVH_LAYOUT_BINARY, _WIDE4 or _WIDE4Q.
 template <bool ANY, int ISECT, bool COUNT, int LAY, class Stack>
 MC_D int trav_step_layout(const TraceScene& sc, TravState& s, const Stack& stack, const WatertightRay& w, int* err,
-                          TravCount* cnt, int cap) {
-    if (LAY == MC_BVH_LAYOUT_WIDE4Q) return trav_step4<ANY, ISECT, COUNT, Stack, true>(sc, s, stack, w, err, cnt, cap);
-    if (LAY == MC_BVH_LAYOUT_WIDE4) return trav_step4<ANY, ISECT, COUNT, Stack, false>(sc, s, stack, w, err, cnt, cap);
-    return trav_step<ANY, ISECT, COUNT, Stack>(sc, s, stack, w, err, cnt, cap);
+                          TravCount* cnt) {
+    if (LAY == MC_BVH_LAYOUT_WIDE4Q) return trav_step4<ANY, ISECT, COUNT, Stack, true>(sc, s, stack, w, err, cnt);
+    if (LAY == MC_BVH_LAYOUT_WIDE4) return trav_step4<ANY, ISECT, COUNT, Stack, false>(sc, s, stack, w, err, cnt);
+    return trav_step<ANY, ISECT, COUNT, Stack>(sc, s, stack, w, err, cnt);
 }
 
 // The hit record fields a leaf slot stands for.
 MC_D void leaf_identity(const TraceScene& sc, int k, int& type, int& id) {
-    float4 c = ldg4(sc.prims + (long long)k * 3 + 2);
+    float4 c = ldg4(leaf_record(sc, k) + 2);
     id = __float_as_int(c.y);
     type = __float_as_int(c.z);
 }
