@@ -64,7 +64,7 @@ mc_status upload_host(mc_context* ctx, void* dst, const void* src, size_t bytes)
 
 // Per-bounce counters of one sample: [d][0] extend-queue size of bounce d,
 // [d][1] shadow-queue size of bounce d, [d][2] trace work counter,
-// [d][3] medium pass-through count.
+// [d][3] work counter of the few-paths kernel.
 #define MC_COUNTERS_PER_DEPTH 4
 
 struct WaveBuffers {
@@ -125,6 +125,8 @@ struct mc_context {
     int trace_blocks[144] = {};
     int trace_blocks_smem[144] = {};     // shared-memory bytes trace_blocks[k] was measured with
     int trace_smem_attr[144] = {};       // dynamic shared memory the variant has been opted in to
+    int paths_blocks[6] = {};            // k_paths: RNG x layout
+    int paths_blocks_smem = 0;           // shared-memory bytes they were measured with
     int shade_blocks[3] = {};            // Philox, XORWOW, guided
     bool guide_attrs_set = false;        // the guide kernels' shared-memory opt-in is done
 };

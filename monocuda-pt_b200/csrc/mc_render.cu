@@ -556,14 +556,28 @@ MC_D void train_remainder(const ShadeArgs& a, int p, int depth, const V3& L, flo
     r[11] = (L.x + L.y + L.z) * (1.0f / 3.0f) * (1.0f - w);
 }
 
+// Dot product with its contraction written out: left to the compiler, which of
+// the first two products is rounded follows how often each is used in the code
+// around the call, so the same shading would round differently in k_shade and
+// k_paths. These are the choices it made for k_shade, whose XORWOW instance
+// differs from the Philox one in the diffuse density only.
+MC_D float shade_dot(const V3& u, const V3& v) { return __fmaf_rn(u.z, v.z, __fmaf_rn(u.y, v.y, __fmul_rn(u.x, v.x))); }
+template <class Rng>
+MC_D float diffuse_dot(const V3& u, const V3& v) {
+    return shade_dot(u, v);
+}
+template <>
+MC_D float diffuse_dot<XorwowRng>(const V3& u, const V3& v) {
+    return __fmaf_rn(u.z, v.z, __fmaf_rn(u.x, v.x, __fmul_rn(u.y, v.y)));
+}
+
 // PT:3470-3696 shadeKernel for one path. GUIDED: diffuse vertices sample the
 // next direction by one-sample MIS of the cosine lobe and the guide. ALIAS:
 // scenes with an alias table draw environment directions from it; the
 // variant without it compiles the reference's CDF sampling on its own, so
 // the image-parity path keeps exactly the reference's instruction sequence.
 template <class Rng, bool GUIDED, bool ALIAS = false>
-MC_D void shade_path(const ShadeArgs& a, const SceneGPU& S, int p, ShadeOut& out) {
-    const int depth = a.depth;
+MC_D void shade_path(const ShadeArgs& a, const SceneGPU& S, int p, int depth, ShadeOut& out) {
     V3 throughput(a.tr[p], a.tg[p], a.tb[p]);
     V3 cs(a.sr[p], a.sg[p], a.sb[p]);
     int4 hraw = reinterpret_cast<const int4*>(a.hits)[p];
@@ -631,7 +645,7 @@ MC_D void shade_path(const ShadeArgs& a, const SceneGPU& S, int p, ShadeOut& out
         float emissionWeight = 1.0f;
         bool fromBsdf = !(depth == 0 || prevSpec);
         if (fromBsdf && ptype == 1) {
-            float cosL = fmaxf(fabsf(inDir.dot(hitNormal)), 1e-4f);
+            float cosL = fmaxf(fabsf(shade_dot(inDir, hitNormal)), 1e-4f);
             float area = triangle_area(tv0, tv1, tv2);
             float lightPdf = light_solid_angle_pdf((1.0f - env_selection_probability(S.env, lightCount)) / float(lightCount),
                                                    hitT, cosL, area);
@@ -694,9 +708,9 @@ MC_D void shade_path(const ShadeArgs& a, const SceneGPU& S, int p, ShadeOut& out
             solidPdf = (cosL > 1e-4f) ? sel * (dist * dist) / (cosL * L.area) : 0.0f;
         }
         bool iso = (mat.type == MC_MAT_ISOTROPIC);
-        float cosS = iso ? 1.0f : hitNormal.dot(toLight);
+        float cosS = iso ? 1.0f : shade_dot(hitNormal, toLight);
         if (cosS > 0.0f && solidPdf > 0.0f) {
-            float phasePdf = hg_phase_pdf(inDir.dot(toLight), mat.g);
+            float phasePdf = hg_phase_pdf(shade_dot(inDir, toLight), mat.g);
             float scatterPdf = iso ? phasePdf : lambertian_cosine_pdf(cosS);
             if (GUIDED && !iso && mat.type == MC_MAT_LAMBERTIAN)
                 scatterPdf = guided_pdf(a.mix + (size_t)mix_path(a, S, p) * guide::kOut, a.guideFrac, hitNormal, toLight, a.fold != 0);
@@ -793,9 +807,9 @@ MC_D void shade_path(const ShadeArgs& a, const SceneGPU& S, int p, ShadeOut& out
         a.tg[p] = throughput.y;
         a.tb[p] = throughput.z;
         a.spec[p] = (mat.type != MC_MAT_LAMBERTIAN && mat.type != MC_MAT_ISOTROPIC) ? 1 : 0;
-        a.pdf[p] = (mat.type == MC_MAT_ISOTROPIC) ? hg_phase_pdf(inDir.dot(nd), mat.g)
+        a.pdf[p] = (mat.type == MC_MAT_ISOTROPIC) ? hg_phase_pdf(shade_dot(inDir, nd), mat.g)
                    : (GUIDED && mat.type == MC_MAT_LAMBERTIAN) ? guidedPdf
-                                                               : lambertian_cosine_pdf(fmaxf(nd.dot(hitNormal), 0.0f));
+                                                               : lambertian_cosine_pdf(fmaxf(diffuse_dot<Rng>(nd, hitNormal), 0.0f));
         out.next = depth + 1 < S.maxDepth;  // the scene's max depth ends the path (PT:3793)
     }
     rng_store<Rng>(a, S, p, rng);
@@ -853,7 +867,7 @@ __global__ void __launch_bounds__(256, GUIDED ? MC_GUIDED_SHADE_BLOCKS : MC_SHAD
                     r[15] = 0.0f;
                 }
             }
-            shade_path<Rng, GUIDED, ALIAS>(a, S, p, out);
+            shade_path<Rng, GUIDED, ALIAS>(a, S, p, a.depth, out);
         }
         int ns = warp_reserve(out.shadow, a.shCount, ltmask);
         if (out.shadow) {
@@ -1214,6 +1228,181 @@ __global__ void __launch_bounds__(256) k_ratio_track(ShadeArgs a, RatioArgs v) {
     }
 }
 
+// Few paths: each lane carries a path from bounce `depth` to its end (closest
+// hit, shading, the shadow ray, the next bounce), in the order and with the
+// arithmetic of the wave's separate launches, so images and random draws are
+// the same. A wave pays a trace and a shade launch per bounce, each as long as
+// its slowest ray; with too few paths to fill the GPU that latency is all there
+// is, and here a path waits for its own rays only: a 64x48 preview 278 -> 164 us,
+// the 333x180 cloud frame of depth 1000 39.1 -> 11.0 ms. Launched where
+// kPathsInFlight says.
+// Lanes per warp as in k_trace: one path per warp when there are few. What the
+// wave passes through memory (a shadow ray's contribution and length) is rounded
+// there, so its uses here are written with explicit roundings.
+struct PathsArgs {
+    const int* queue;
+    const int* count;
+    int* work;
+    int stackCap;
+    int gridMedia;       // the wave's trace launches would be the density-grid variant
+    int depth;           // bounce the queued paths are at
+    long long* stats;    // extend and shadow rays per depth
+    int* err;
+};
+
+constexpr int kPathsThreads = 128;
+
+MC_D void opaque(float& x) { asm volatile("" : "+f"(x)); }
+MC_D void opaque(V3& v) {
+    opaque(v.x);
+    opaque(v.y);
+    opaque(v.z);
+}
+
+template <bool ANY, int LAY, class Stack>
+MC_D int trace_to_end(const TraceScene& ts, TravState& s, const Stack& stack, int* err) {
+    const WatertightRay w{};
+    TravCount cnt;
+    int r;
+    do r = trav_step_layout<ANY, MC_ISECT_REFERENCE, false, LAY>(ts, s, stack, w, err, &cnt);
+    while (r == STEP_CONTINUE);
+    return r;
+}
+
+// The transmittance of a shadow ray (PT:2874-2898; finish_ray and
+// k_ratio_track in one): 0 when blocked.
+template <class Rng, int LAY, class Stack>
+MC_D float shadow_ray(const ShadeArgs& a, const PathsArgs& v, const SceneGPU& S, const TraceScene& ts, const Stack& stack,
+                      int p, const ShadeOut& out) {
+    TravState s;
+    const float time = a.time[p];
+    trav_begin(s, stack, out.so, out.sd, time, out.smax, ts.root);
+    if (!S.hasMedium) return trace_to_end<true, LAY>(ts, s, stack, v.err) == STEP_OCCLUDED ? 0.0f : 1.0f;
+    float T = 1.0f, travelled = 0.0f;
+    if (out.smax <= 0.0f) return T;
+    bool drawn = false, blocked = false;
+    Rng rng;
+    for (int crossings = 0;;) {
+        trace_to_end<false, LAY>(ts, s, stack, v.err);
+        if (s.hitLeaf < 0) break;
+        int type, id;
+        leaf_identity(ts, s.hitLeaf, type, id);
+        const mc_material* m = type == 1 ? &S.cold[id].mat : &S.spheres[id].mat;
+        if (m->type != MC_MAT_ISOTROPIC) {
+            blocked = true;
+            break;
+        }
+        bool front;
+        if (type == 1) {
+            const float4 n4 = ldg4(leaf_record(ts, s.hitLeaf) + 3);
+            front = s.r.d.dot(V3(n4.x, n4.y, n4.z)) < 0.0f;
+        } else {
+            const mc_sphere& sp = S.spheres[id];
+            float tt;
+            V3 outward;
+            hit_sphere_ref(v3(sp.center), v3(sp.center1), sp.is_moving != 0, sp.radius, s.r.o, s.r.d, s.time, tt, front,
+                           outward);
+        }
+        if (!front) {
+            if (v.gridMedia && m->density_grid) {
+                if (!drawn) rng_load<Rng>(a, S, p, rng);
+                drawn = true;
+                T = T * volume_transmittance(static_cast<const mc_volume_grid*>(m->density_grid), m->density,
+                                             m->grid_max_density, s.r.o, s.r.d, s.tmax, rng);
+            } else {
+                T = T * expf(-m->density * s.tmax);
+            }
+        }
+        travelled = travelled + s.tmax;
+        V3 hp = s.r.o + s.r.d * s.tmax;
+        const float remaining = __fadd_rn(out.smax, -travelled);
+        if (++crossings >= 4 || remaining <= 0.0f) break;
+        s.r.o = hp;
+        trav_restart(s, stack, remaining, ts.root);
+    }
+    if (drawn) rng_store<Rng>(a, S, p, rng);
+    return blocked ? 0.0f : T;
+}
+
+template <class Rng, int LAY>
+__global__ void __launch_bounds__(kPathsThreads) k_paths(ShadeArgs a, PathsArgs v) {
+    extern __shared__ int traceStack[];
+    const SharedStack<kPathsThreads> stack(traceStack, v.stackCap);
+    const int lane = threadIdx.x & 31;
+    const unsigned ltmask = lanemask_lt();
+    const int total = min(*v.count, a.capacity);
+    const int warps = gridDim.x * (kPathsThreads / 32);
+    const int width = min(32, (total + warps - 1) / warps);
+    bool exhausted = total == 0;
+    int p = -1, depth = 0;
+    while (true) {
+        const unsigned idle = __ballot_sync(kFull, p < 0);
+        const int take = width - (32 - __popc(idle));
+        if (!exhausted && take > 0) {
+            const int leader = __ffs(idle) - 1;
+            int base = 0;
+            if (lane == leader) base = atomicAdd(v.work, take);
+            base = __shfl_sync(kFull, base, leader);
+            const int nth = __popc(idle & ltmask);
+            if (p < 0 && nth < take && base + nth < total) {
+                p = v.queue[base + nth];
+                depth = v.depth;
+            }
+            if (base + take >= total) exhausted = true;
+        }
+        if (__ballot_sync(kFull, p >= 0) == 0u) {
+            if (exhausted) break;
+            continue;
+        }
+        if (p >= 0) {
+            const SceneGPU& S = a.tab->scenes[scene_of(a.tab, a.sceneOf, p)];
+            TraceScene ts;
+            ts.nodes = S.nodes;
+            ts.prims = S.prims;
+            ts.root = S.root;
+            const int bucket = min(depth, MC_MAX_DEPTH_STATS - 1);
+            // the first bounce's extend rays are in the wave's counters already
+            if (depth != v.depth) atomicAdd((unsigned long long*)&v.stats[bucket], 1ull);
+            {
+                TravState s;
+                trav_begin(s, stack, V3(a.ox[p], a.oy[p], a.oz[p]), V3(a.dx[p], a.dy[p], a.dz[p]), a.time[p], 1e30f, ts.root);
+                trace_to_end<false, LAY>(ts, s, stack, v.err);
+                int type = -1, id = -1, did = 0;
+                if (s.hitLeaf >= 0) {
+                    leaf_identity(ts, s.hitLeaf, type, id);
+                    did = 1;
+                }
+                reinterpret_cast<int4*>(const_cast<mc_packed_hit*>(a.hits))[p] = make_int4(__float_as_int(s.tmax), type, id, did);
+            }
+            // the shading sees the path state as its own kernel does, from memory,
+            // and hands its results over as values: nothing of the code around it
+            // takes part in its arithmetic
+            int q = p;
+            asm volatile("" : "+r"(q) : : "memory");
+            ShadeOut out;
+            out.next = false;
+            out.shadow = false;
+            shade_path<Rng, false>(a, S, q, depth, out);
+            asm volatile("" : : : "memory");
+            if (out.shadow) {
+                opaque(out.so);
+                opaque(out.sd);
+                opaque(out.contrib);
+                opaque(out.smax);
+                atomicAdd((unsigned long long*)&v.stats[MC_MAX_DEPTH_STATS + bucket], 1ull);
+                const float T = shadow_ray<Rng, LAY>(a, v, S, ts, stack, p, out);
+                if (T > 0.0f) {
+                    a.sr[p] = __fmaf_rn(out.contrib.x, T, a.sr[p]);
+                    a.sg[p] = __fmaf_rn(out.contrib.y, T, a.sg[p]);
+                    a.sb[p] = __fmaf_rn(out.contrib.z, T, a.sb[p]);
+                }
+            }
+            depth++;
+            if (!out.next) p = -1;
+        }
+    }
+}
+
 // Renders deeper than the counter block (max_depth > MC_MAX_DEPTH_STATS) use
 // its MC_MAX_DEPTH_STATS + 1 slots as a ring: bounce d's counters live in
 // slot d % kRingSlots. Before bounce d + kRingSlots reuses a slot, its counts
@@ -1475,6 +1664,34 @@ static void set_single_scene(TraceArgs& t, const mc_bvh* bvh, int root, const mc
     t.spheres0 = v->spheres;
 }
 
+// Waves of at most this many paths run as one k_paths launch, and deep waves
+// (max_depth > MC_MAX_DEPTH_STATS) hand their paths over once so few go on.
+// Where the line lies (paths: wave launches / one launch, us): Cornell boxes
+// 4,096: 298 / 189, 65,536: 372 / 355, 131,044: 436 / 479; spheres, depth 20,
+// 4,096: 472 / 243, 65,536: 726 / 684, 131,044: 857 / 985; icospheres (246k
+// triangles) 883 / 817 and 1043 / 1037. With density grids a bounce waits on
+// long chains of voxel reads and every path on its own: 131,044 paths of the
+// cloud 65,800 / 15,100, 960k 26,100 (handed over at 65,536) / 20,700.
+constexpr int kPathsInFlight = 1 << 16;
+constexpr int kPathsInFlightGrid = 1 << 20;
+
+static void launch_paths(mc_context* ctx, cudaStream_t stream, const ShadeArgs& a, PathsArgs v, int layout, bool philox) {
+    typedef void (*Kernel)(ShadeArgs, PathsArgs);
+    static const Kernel table[2][3] = {{k_paths<PhiloxRng, 0>, k_paths<PhiloxRng, 1>, k_paths<PhiloxRng, 2>},
+                                       {k_paths<XorwowRng, 0>, k_paths<XorwowRng, 1>, k_paths<XorwowRng, 2>}};
+    const Kernel fn = table[philox ? 0 : 1][layout];
+    if (v.stackCap <= 0 || v.stackCap > MC_STACK_CAPACITY) v.stackCap = MC_STACK_CAPACITY;
+    const int smem = kPathsThreads * v.stackCap * (int)sizeof(int);  // at most 32 KB: no opt-in
+    int& blocks = ctx->paths_blocks[(philox ? 0 : 3) + layout];
+    if (!blocks || ctx->paths_blocks_smem != smem) {
+        if (ctx->paths_blocks_smem != smem)
+            for (int& b : ctx->paths_blocks) b = 0;
+        blocks = occupancy_blocks((const void*)fn, ctx->sm_count, smem, kPathsThreads);
+        ctx->paths_blocks_smem = smem;
+    }
+    fn<<<blocks, kPathsThreads, smem, stream>>>(a, v);
+}
+
 // Levels of a greedy 4-wide tree, -1 for other trees.
 static int shape_levels(const mc_bvh* b) { return b->layout == MC_BVH_LAYOUT_BINARY || b->wide_levels <= 0 ? -1 : b->wide_levels; }
 
@@ -1664,6 +1881,27 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
     // paths, the same primary ray) share one inference
     const bool shareMix = guide && n == 1;
     if (guide && train && guidedDepth > 0) guidedDepth = std::max(guidedDepth, guide->cfg.train_vertices + 1);
+    // launches of k_paths: not where a variant of the wave's own kernels was
+    // asked for (instruments, the watertight test, alias sampling, a queue
+    // limit, the plain mode)
+    const bool pathsOk = !guide && !timeTrace && !countVisits && !alias && isect == MC_ISECT_REFERENCE && persistent &&
+                         p0.queue_capacity == 0 && maxD > 0;
+    const int fewPaths = grid ? kPathsInFlightGrid : kPathsInFlight;
+    const bool smallWave = pathsOk && capacity <= fewPaths;
+    auto enqueue_paths = [&](int d) {
+        PathsArgs v;
+        std::memset(&v, 0, sizeof(v));
+        v.queue = w.queue[d & 1];
+        v.count = slot(d) + 0;
+        v.work = slot(d) + 3;
+        v.stackCap = ta.stackCap;
+        v.gridMedia = grid ? 1 : 0;
+        v.depth = d;
+        v.stats = ctx->d_stats;
+        v.err = ctx->d_error;
+        launch_paths(ctx, stream, sa, v, layout, philox);
+        launches++;
+    };
     auto enqueue_wave = [&]() -> mc_status {
         MC_CUDA(cudaMemsetAsync(C, 0, counterBytes, stream));
         if (guide) {
@@ -1673,9 +1911,15 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
         if (philox) k_camera<PhiloxRng><<<loopBlocks, 256, 0, stream>>>(ca);
         else k_camera<XorwowRng><<<loopBlocks, 256, 0, stream>>>(ca);
         launches++;
-        int dEnd = maxD;
-        bool stop = false;
-        for (int d = 0; d <= maxD; d++) {
+        int dEnd = maxD;     // depths [0, dEnd) have counts in the counter slots
+        int dLast = maxD;    // the last bounce with launches of its own
+        bool stop = false, few = false;  // few: the remaining paths go to k_paths
+        if (smallWave) {
+            enqueue_paths(0);
+            dLast = 0;
+            dEnd = 1;
+        }
+        for (int d = 0; d <= maxD && !smallWave; d++) {
             const bool last = d == maxD || stop;  // shadow rays of the previous bounce only
             TraceArgs t = ta;
             if (!last) {
@@ -1707,7 +1951,11 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
                 launches++;
             }
             if (last) {
-                dEnd = d;
+                dLast = dEnd = d;
+                if (few) {
+                    enqueue_paths(d);
+                    dEnd = d + 1;
+                }
                 break;
             }
             // bounces past the guided depth shade with the cosine lobe alone: no inference
@@ -1765,7 +2013,8 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
                 int next = 0;
                 MC_CUDA(cudaMemcpyAsync(&next, slot(d + 1), sizeof(int), cudaMemcpyDeviceToHost, stream));
                 MC_CUDA(cudaStreamSynchronize(stream));
-                stop = next == 0;
+                few = pathsOk && next > 0 && next <= fewPaths;
+                stop = next == 0 || few;
             }
         }
         if (guide) {
@@ -1791,8 +2040,8 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
         } else {
             k_finalize<<<loopBlocks, 256, 0, stream>>>(dtab, w.sr, w.sg, w.sb);
         }
-        if (deep) k_accumulate_ring<<<1, 32, 0, stream>>>(C, std::max(0, dEnd - (kRingSlots - 1)), dEnd, ctx->d_stats);
-        else k_accumulate_counts<<<1, 64, 0, stream>>>(C, maxD, ctx->d_stats);
+        if (deep) k_accumulate_ring<<<1, 32, 0, stream>>>(C, std::max(0, dLast - (kRingSlots - 1)), dEnd, ctx->d_stats);
+        else k_accumulate_counts<<<1, 64, 0, stream>>>(C, smallWave ? dEnd : maxD, ctx->d_stats);
         launches += 2;
         if (guide && train) {
             // as many Adam steps per sample, on as many records each, as with
@@ -1817,7 +2066,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
                                       (unsigned long long)maxD,
                                       (unsigned long long)((layout << 6) | (medium ? 2 : 0) | (philox ? 4 : 0) |
                                                            (persistent ? 8 : 0) | (n > 1 ? 16 : 0) |
-                                                           (sameScene ? 32 : 0) | (grid ? 1024 : 0)),
+                                                           (sameScene ? 32 : 0) | (grid ? 1024 : 0) | (smallWave ? 2048 : 0)),
                                       (unsigned long long)isect,
                                       (unsigned long long)ta.refill,
                                       (unsigned long long)(uintptr_t)ta.ts0.nodes,
@@ -1892,7 +2141,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
         MC_CUDA(cudaEventRecord((cudaEvent_t)ctx->table_events[slot], stream));
         if (useGraph) {
             MC_CUDA(cudaGraphLaunch(exec, stream));
-            perWave = 3 + 2 * maxD + (grid ? maxD : 0);
+            perWave = smallWave ? 4 : 3 + 2 * maxD + (grid ? maxD : 0);
         } else {
             if ((st = enqueue_wave()) != MC_OK) return st;
         }
