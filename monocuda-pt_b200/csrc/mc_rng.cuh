@@ -60,10 +60,13 @@ struct PhiloxRng {
         draw++;
         return word_to_uniform(w);
     }
+    static constexpr bool kGivesBack = true;
+    MC_D void give_back(int n) { draw -= (uint32_t)n; }  // the last n draws were not taken
 };
 
 struct XorwowRng {
     curandState st;
+    static constexpr bool kGivesBack = false;
     MC_D float uniform() { return curand_uniform(&st); }
 };
 
