@@ -112,18 +112,24 @@ mc_status mc_render_host(mc_context* ctx, const mc_triangle* tris, int32_t n_tri
         return mc::set_error(MC_ERR_INVALID, "mc_render_host: bad argument");
     if (n_tri + n_sph == 0) return mc::set_error(MC_ERR_INVALID, "mc_render_host: the scene has no primitives");
     const size_t nt = (size_t)(n_tri > 0 ? n_tri : 1);
-    mc_triangle_hot* dHot = nullptr; mc_triangle_cold* dCold = nullptr; mc_sphere* dSph = nullptr; mc_light* dL = nullptr;
-    float* dAcc = nullptr;
-    size_t accBytes = (size_t)params->width * params->height * 3 * sizeof(float);
-    auto cleanup = [&]() { cudaFree(dHot); cudaFree(dCold); cudaFree(dSph); cudaFree(dL); cudaFree(dAcc); };
-    if (cudaMalloc(&dHot, nt * sizeof(mc_triangle_hot)) != cudaSuccess ||
-        cudaMalloc(&dCold, nt * sizeof(mc_triangle_cold)) != cudaSuccess ||
-        cudaMalloc(&dSph, (size_t)(n_sph > 0 ? n_sph : 1) * sizeof(mc_sphere)) != cudaSuccess ||
-        cudaMalloc(&dL, nt * sizeof(mc_light)) != cudaSuccess || cudaMalloc(&dAcc, accBytes) != cudaSuccess) {
-        cudaGetLastError();
-        cleanup();
-        return mc::set_error(MC_ERR_OOM, "mc_render_host: device allocation failed");
-    }
+    const size_t accBytes = (size_t)params->width * params->height * 3 * sizeof(float);
+    const size_t size[5] = {nt * sizeof(mc_triangle_hot), nt * sizeof(mc_triangle_cold),
+                            (size_t)(n_sph > 0 ? n_sph : 1) * sizeof(mc_sphere), nt * sizeof(mc_light), accBytes};
+    void* buf[5] = {};
+    auto cleanup = [&]() {
+        for (int i = 0; i < 5; i++)
+            if (buf[i]) mc::call_free(ctx, buf[i], size[i]);
+    };
+    for (int i = 0; i < 5; i++)
+        if (mc::call_alloc(ctx, &buf[i], size[i]) != MC_OK) {
+            cleanup();
+            return mc::set_error(MC_ERR_OOM, "mc_render_host: device allocation failed");
+        }
+    mc_triangle_hot* dHot = (mc_triangle_hot*)buf[0];
+    mc_triangle_cold* dCold = (mc_triangle_cold*)buf[1];
+    mc_sphere* dSph = (mc_sphere*)buf[2];
+    mc_light* dL = (mc_light*)buf[3];
+    float* dAcc = (float*)buf[4];
     if (n_sph) cudaMemcpyAsync(dSph, spheres, (size_t)n_sph * sizeof(mc_sphere), cudaMemcpyHostToDevice, ctx->stream);
     cudaMemcpyAsync(dAcc, accum_host, accBytes, cudaMemcpyHostToDevice, ctx->stream);
     int32_t nl = 0, hasMedium = 0;

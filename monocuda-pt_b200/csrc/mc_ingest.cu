@@ -257,13 +257,13 @@ extern "C" mc_status mc_scene_ingest_host(mc_context* ctx, const mc_triangle* tr
                                           int32_t* light_count, int32_t* has_medium) {
     using namespace mc;
     if (!ctx || n < 0 || (n > 0 && !tris)) return set_error(MC_ERR_INVALID, "mc_scene_ingest_host: bad arguments");
-    mc_triangle* dTri = nullptr;
-    if (n > 0 && cudaMalloc(&dTri, (size_t)n * sizeof(mc_triangle)) != cudaSuccess) {
-        cudaGetLastError();
-        return set_error(MC_ERR_OOM, "mc_scene_ingest_host: device allocation failed");
-    }
-    mc_status st = upload_host(ctx, dTri, tris, (size_t)n * sizeof(mc_triangle));
-    if (st == MC_OK) st = mc_scene_ingest(ctx, dTri, n, spheres, n_sph, hot, cold, lights, light_count, has_medium);
-    cudaFree(dTri);
+    void* dTri = nullptr;
+    const size_t bytes = (size_t)n * sizeof(mc_triangle);
+    mc_status st = MC_OK;
+    if (n > 0 && (st = call_alloc(ctx, &dTri, bytes)) != MC_OK) return st;
+    st = upload_host(ctx, dTri, tris, bytes);
+    if (st == MC_OK)
+        st = mc_scene_ingest(ctx, (const mc_triangle*)dTri, n, spheres, n_sph, hot, cold, lights, light_count, has_medium);
+    call_free(ctx, dTri, bytes);
     return st;
 }

@@ -55,6 +55,9 @@ void devbuf_free(DevBuf& b);
 mc_status pool_alloc(mc_context* ctx, void** p, size_t bytes);
 void pool_free(mc_context* ctx, void* p);  // ordered after the work queued on ctx's stream
 void pool_release(void* p);                // device current and its readers finished
+// a call's own buffers: pooled when small, else cudaMalloc / cudaFree
+mc_status call_alloc(mc_context* ctx, void** p, size_t bytes);
+void call_free(mc_context* ctx, void* p, size_t bytes);
 void pool_trim(int device);                // hands the pool's unused memory back
 
 // Copies `bytes` of host memory to the device; complete when the call returns.
