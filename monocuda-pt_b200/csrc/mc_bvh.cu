@@ -158,9 +158,18 @@ __global__ void k_prim_bounds(const Seg* __restrict__ seg, int nseg, int n, mc_a
         bounds[g] = a;
         centroids[g] = make_float4(cx, cy, cz, __int_as_float(s));
     }
+    // Scene bounds: one set of words per scene that every primitive may have to
+    // lower or raise. A block reduces its primitives first (a warp, where the
+    // block holds several scenes), and a word that is already past the value is
+    // left alone: per-warp atomics without either took 110 of this kernel's
+    // 130 us at 1M triangles.
     int* sb = scene + 6 * s;
-    int s0 = __shfl_sync(0xffffffffu, s, 0);
-    if (__all_sync(0xffffffffu, s == s0)) {
+    __shared__ Box warpBox[kBlock / 32];
+    const int first = __shfl_sync(0xffffffffu, s, 0);
+    const bool warpSame = __all_sync(0xffffffffu, !valid || s == first);
+    const int blockFirst = seg_of_prim(seg, nseg, min(blockIdx.x * (int)blockDim.x, n - 1));
+    const bool blockSame = __syncthreads_and(!valid || s == blockFirst);
+    if (warpSame) {
         for (int off = 16; off > 0; off >>= 1) {
             b.lx = fminf(b.lx, __shfl_xor_sync(0xffffffffu, b.lx, off));
             b.ly = fminf(b.ly, __shfl_xor_sync(0xffffffffu, b.ly, off));
@@ -169,16 +178,30 @@ __global__ void k_prim_bounds(const Seg* __restrict__ seg, int nseg, int n, mc_a
             b.hy = fmaxf(b.hy, __shfl_xor_sync(0xffffffffu, b.hy, off));
             b.hz = fmaxf(b.hz, __shfl_xor_sync(0xffffffffu, b.hz, off));
         }
-        if ((threadIdx.x & 31) != 0) return;
-    } else if (!valid) {
-        return;
+        if (blockSame) {
+            if ((threadIdx.x & 31) == 0) warpBox[threadIdx.x >> 5] = b;
+            __syncthreads();
+            if (threadIdx.x != 0) return;
+            for (int w = 1; w < kBlock / 32; w++) b = merge_box(b, warpBox[w]);
+        } else if ((threadIdx.x & 31) != 0) {
+            return;
+        }
     }
-    atomicMin(&sb[0], float_to_ordered(b.lx));
-    atomicMin(&sb[1], float_to_ordered(b.ly));
-    atomicMin(&sb[2], float_to_ordered(b.lz));
-    atomicMax(&sb[3], float_to_ordered(b.hx));
-    atomicMax(&sb[4], float_to_ordered(b.hy));
-    atomicMax(&sb[5], float_to_ordered(b.hz));
+    if (!valid) return;
+    auto lower = [](int* word, float f) {
+        const int v = float_to_ordered(f);
+        if (v < __ldcg(word)) atomicMin(word, v);
+    };
+    auto raise = [](int* word, float f) {
+        const int v = float_to_ordered(f);
+        if (v > __ldcg(word)) atomicMax(word, v);
+    };
+    lower(&sb[0], b.lx);
+    lower(&sb[1], b.ly);
+    lower(&sb[2], b.lz);
+    raise(&sb[3], b.hx);
+    raise(&sb[4], b.hy);
+    raise(&sb[5], b.hz);
 }
 
 __global__ void k_init_bounds(int* scene, int nseg) {
@@ -467,7 +490,7 @@ __global__ void k_leaves_refit(const int32_t* __restrict__ order, const mc_aabb*
                                float4* __restrict__ prims, const int32_t* __restrict__ parents, int* __restrict__ counters,
                                int32_t* __restrict__ ids_out, int32_t* __restrict__ types_out,
                                mc_bvh_node* __restrict__ ref_internal, mc_bvh_node* __restrict__ ref_leaves,
-                               mc_aabb* __restrict__ root_boxes, int* __restrict__ err) {
+                               mc_aabb* __restrict__ root_boxes, int* __restrict__ err, bool boxes) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= N) return;
     int src = order[k];
@@ -514,6 +537,7 @@ __global__ void k_leaves_refit(const int32_t* __restrict__ order, const mc_aabb*
         atomicOr(err, MC_DEVERR_INPUT);  // every leaf of a Karras tree over n >= 2 keys has a parent
         return;
     }
+    if (!boxes) return;
     for (int level = 0; p >= 0; level++) {
         int node = p >> 1, side = p & 1;
         if (node >= NI || level > 2 * MC_STACK_CAPACITY) {
@@ -659,9 +683,9 @@ __global__ void k_scatter_ids(const int* __restrict__ roots, int n, int* __restr
 // Count: every wide node of the frontier picks its slots, keeps its internal
 // ones in slot order and adds their number to its tile's total (tile = kBlock
 // frontier entries, one block; warpSum: kBlock / 32 entries).
-__device__ __forceinline__ void wide_count_tile(const float4* nodes, const int* frontier, int n, int capacity,
-                                                const int* wideId, int* rootOf, int4* internal, int* blockTotals, int* err,
-                                                int tile, int* warpSum) {
+__device__ __forceinline__ int wide_count_tile(const float4* nodes, const int* frontier, int n, int capacity,
+                                               const int* wideId, int* rootOf, int4* internal, int* err, int tile,
+                                               int* warpSum) {
     const int i = tile * kBlock + threadIdx.x;
     int nInt = 0;
     if (i < n) {
@@ -683,12 +707,10 @@ __device__ __forceinline__ void wide_count_tile(const float4* nodes, const int* 
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) warpSum[threadIdx.x >> 5] = v;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int k = 0; k < kBlock / 32; k++) t += warpSum[k];
-        blockTotals[tile] = t;
-    }
+    int t = 0;
+    for (int k = 0; k < kBlock / 32; k++) t += warpSum[k];
     __syncthreads();  // warpSum is reused by the block's next tile
+    return t;
 }
 
 __global__ void __launch_bounds__(kBlock) k_wide_level_count(const float4* __restrict__ nodes,
@@ -697,7 +719,8 @@ __global__ void __launch_bounds__(kBlock) k_wide_level_count(const float4* __res
                                                              int4* __restrict__ internal, int* __restrict__ blockTotals,
                                                              int* err) {
     __shared__ int warpSum[kBlock / 32];
-    wide_count_tile(nodes, frontier, n, capacity, wideId, rootOf, internal, blockTotals, err, blockIdx.x, warpSum);
+    const int t = wide_count_tile(nodes, frontier, n, capacity, wideId, rootOf, internal, err, blockIdx.x, warpSum);
+    if (threadIdx.x == 0) blockTotals[blockIdx.x] = t;
 }
 
 // Scan: exclusive prefix of `count` ints in place by one block (a multiple of
@@ -743,8 +766,8 @@ __global__ void __launch_bounds__(1024) k_wide_level_scan(int* blockTotals, int 
 // Write: the internal children of frontier node i take wide ids idBase + o,
 // o = (internal children of the nodes before i), and the same places of the
 // next frontier.
-__device__ __forceinline__ void wide_write_tile(const int4* internal, int n, const int* blockFirst, int idBase,
-                                                int capacity, int* next, int* wideId, int* err, int tile, int* warpSum) {
+__device__ __forceinline__ void wide_write_tile(const int4* internal, int n, int first, int idBase, int capacity,
+                                                int* next, int* wideId, int* err, int tile, int* warpSum) {
     const int i = tile * kBlock + threadIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int4 r = make_int4(-1, -1, -1, -1);
@@ -757,7 +780,7 @@ __device__ __forceinline__ void wide_write_tile(const int4* internal, int n, con
     }
     if (lane == 31) warpSum[wid] = x;
     __syncthreads();
-    int off = blockFirst[tile] + x - nInt;
+    int off = first + x - nInt;
     for (int k = 0; k < wid; k++) off += warpSum[k];
     const int refs[4] = {r.x, r.y, r.z, r.w};
     for (int k = 0; k < nInt; k++) {
@@ -776,14 +799,19 @@ __global__ void __launch_bounds__(kBlock) k_wide_level_write(const int4* __restr
                                                              int capacity, int* __restrict__ next,
                                                              int* __restrict__ wideId, int* err) {
     __shared__ int warpSum[kBlock / 32];
-    wide_write_tile(internal, n, blockFirst, idBase, capacity, next, wideId, err, blockIdx.x, warpSum);
+    wide_write_tile(internal, n, blockFirst[blockIdx.x], idBase, capacity, next, wideId, err, blockIdx.x, warpSum);
 }
 
-// Every level of the collapse in one cooperative launch: the three steps of
-// a level as loops over the same tiles, a grid-wide barrier after each; all
-// blocks read the level's total from the same place after a barrier, so they
-// run the same levels. Ends when a level adds no internal node, after
+// Every level of the collapse in one cooperative launch. Each block takes a
+// contiguous range of a level's tiles: it counts its internal slots, and after a
+// grid-wide barrier adds up the totals of the blocks before it and writes; a
+// second barrier ends the level. Ids follow the frontier's order, as with the
+// per-level launches. Levels of up to kWideOneBlock nodes (the first ones, and
+// the last) run in the first block without grid-wide barriers. Every block reads
+// the same totals, so all run the same levels. With three barriers on every
+// level 1M triangles took 370 us. Ends when a level adds no internal node, after
 // maxLevels + 1 levels, or when the wide ids would pass the node count (error).
+constexpr int kWideOneBlock = 4 * kBlock;
 struct WideLevels {
     const float4* nodes;
     int* front[2];
@@ -791,40 +819,101 @@ struct WideLevels {
     int* wideId;
     int* rootOf;
     int4* internal;
-    int* blockTotals;
-    int* total;
-    int* out;  // [0] levels, [1] wide nodes, [2] last frontier size, [3] 1 when the ids would pass capacity
+    int* tileFirst;    // per tile: internal slots of its block's earlier tiles
+    int* blockTotals;  // per block
+    int* out;          // [0] levels, [1] wide nodes, [2] last frontier size, [3] 1 when the ids would pass capacity, [4] buffer
     int* err;
 };
 
 __global__ void __launch_bounds__(kBlock) k_wide_levels(WideLevels a) {
     cooperative_groups::grid_group grid = cooperative_groups::this_grid();
     __shared__ int warpSum[32];
-    __shared__ int carry;
+    __shared__ int sBefore, sTotal;
     int n = a.nseg, idBase = a.nseg, cur = 0, levels = 0;
     bool bad = false;
-    while (n > 0 && levels <= a.maxLevels) {
-        const int* front = cur ? a.front[1] : a.front[0];
-        int* next = cur ? a.front[0] : a.front[1];
-        const int tiles = (n + kBlock - 1) / kBlock;
-        for (int t = blockIdx.x; t < tiles; t += gridDim.x)
-            wide_count_tile(a.nodes, front, n, a.capacity, a.wideId, a.rootOf, a.internal, a.blockTotals, a.err, t,
-                            warpSum);
-        grid.sync();
-        if (blockIdx.x == 0) scan_ints_block(a.blockTotals, tiles, a.total, warpSum, carry);
-        grid.sync();
-        for (int t = blockIdx.x; t < tiles; t += gridDim.x)
-            wide_write_tile(a.internal, n, a.blockTotals, idBase, a.capacity, next, a.wideId, a.err, t, warpSum);
-        grid.sync();
-        const int m = *a.total;  // written by block 0 before the last barrier
+    auto count_range = [&](int t0, int t1) {
+        int carry = 0;
+        for (int t = t0; t < t1; t++) {
+            const int c = wide_count_tile(a.nodes, cur ? a.front[1] : a.front[0], n, a.capacity, a.wideId, a.rootOf,
+                                          a.internal, a.err, t, warpSum);
+            if (threadIdx.x == 0) a.tileFirst[t] = carry;
+            carry += c;
+        }
+        __syncthreads();
+        return carry;
+    };
+    auto write_range = [&](int t0, int t1, int before) {
+        for (int t = t0; t < t1; t++)
+            wide_write_tile(a.internal, n, before + a.tileFirst[t], idBase, a.capacity, cur ? a.front[0] : a.front[1], a.wideId,
+                            a.err, t, warpSum);
+    };
+    auto advance = [&](int m) {
         if (m < 0 || (long long)idBase + m > a.capacity) {
             bad = true;
-            break;
+            return;
         }
         idBase += m;
         n = m;
         cur = 1 - cur;
         levels++;
+    };
+    auto level_alone = [&]() {
+        const int tiles = (n + kBlock - 1) / kBlock;
+        const int m = count_range(0, tiles);
+        write_range(0, tiles, 0);
+        __syncthreads();
+        advance(m);
+    };
+    if (blockIdx.x == 0) {
+        while (n > 0 && n <= kWideOneBlock && levels <= a.maxLevels && !bad) level_alone();
+        if (threadIdx.x == 0) {
+            a.out[0] = levels;
+            a.out[1] = idBase;
+            a.out[2] = n;
+            a.out[3] = bad ? 1 : 0;
+            a.out[4] = cur;
+        }
+    }
+    grid.sync();
+    levels = __ldcg(&a.out[0]);
+    idBase = __ldcg(&a.out[1]);
+    n = __ldcg(&a.out[2]);
+    bad = __ldcg(&a.out[3]) != 0;
+    cur = __ldcg(&a.out[4]);
+    while (n > 0 && levels <= a.maxLevels && !bad) {
+        if (n <= kWideOneBlock) {
+            if (blockIdx.x != 0) return;
+            level_alone();
+            continue;
+        }
+        const int tiles = (n + kBlock - 1) / kBlock;
+        const int t0 = (int)((long long)tiles * blockIdx.x / gridDim.x);
+        const int t1 = (int)((long long)tiles * (blockIdx.x + 1) / gridDim.x);
+        const int mine = count_range(t0, t1);
+        if (threadIdx.x == 0) {
+            a.blockTotals[blockIdx.x] = mine;
+            sBefore = sTotal = 0;
+        }
+        grid.sync();
+        int before = 0, total = 0;
+        for (int k = threadIdx.x; k < (int)gridDim.x; k += kBlock) {
+            const int c = __ldcg(&a.blockTotals[k]);
+            total += c;
+            if (k < (int)blockIdx.x) before += c;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            before += __shfl_xor_sync(0xffffffffu, before, o);
+            total += __shfl_xor_sync(0xffffffffu, total, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(&sBefore, before);
+            atomicAdd(&sTotal, total);
+        }
+        __syncthreads();
+        const int m = sTotal;
+        write_range(t0, t1, sBefore);
+        grid.sync();
+        advance(m);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.out[0] = levels;
@@ -1497,38 +1586,109 @@ __global__ void k_ploc_advance(const int2* __restrict__ total, int* __restrict__
     state[0] = t.y;
 }
 
-// Every clustering round in one cooperative launch. A round's phases (nearest
-// neighbours, merge flags, tile scans, the scan of the tile sums by block 0,
-// emit) take the same tiles as the per-phase launches above, as grid-stride
-// loops, with a grid-wide barrier after each; every block reads the round's
-// totals from the same place after a barrier, so all blocks run the same
-// rounds and reach the same barriers, and the tree is the per-phase launches'
-// to the bit. The loop ends when every scene is one cluster, after maxRounds
-// rounds (error), or when a round merges nothing (error: the globally closest
-// pair is always mutual).
+// Every clustering round in one cooperative launch. The positions of a round
+// are cut into tiles of kPlocBlock, each block takes a contiguous range of
+// tiles, and a round is two phases with a grid-wide barrier after each:
+//   1. nearest neighbours of the tile and of kPlocRadius positions on either
+//      side (so that whether a pair is mutual is known without asking another
+//      block), merge and survival flags, and the places of the tile's merges
+//      and survivors among the block's;
+//   2. the block's place among the blocks (each sums the totals before its
+//      own), then the new nodes and the compacted clusters.
+// Merges and survivors keep the order of positions, so the tree is that of the
+// per-phase launches above to the bit. Most rounds hold few clusters (a scene's
+// large triangles join one or two a round) and cost their barriers: the last
+// ones, of up to kPlocOneBlock positions, run in the first block alone. Five
+// barriers a round and none of this took 990 us for 1M triangles. The loop ends
+// when every scene is one cluster, after maxRounds rounds (error), or when a
+// round merges nothing (error: the globally closest pair is always mutual);
+// every block computes the same totals, so all run the same rounds and barriers.
+constexpr int kPlocOneBlock = 4 * kPlocBlock;
 struct PlocRounds {
     int* cref[2];
     float4* cbox[2];
     int* nn;
-    int2* flags;
     int2* pos;
-    int2* sums;
-    int2* total;
+    int2* sums;  // per block: merges and survivors of its range
     int* state;  // out: [0] clusters left, [1] internal nodes written, [2] buffer of the last clusters, [3] rounds
     float4* nodes;
     int nodeCap, nseg, N, maxRounds;
     int* err;
 };
 
+struct PlocShared {
+    static constexpr int kWindow = kPlocBlock + 4 * kPlocRadius;
+    static constexpr int kNear = kPlocBlock + 2 * kPlocRadius;
+    float4 lo[kWindow], hi[kWindow];
+    int near[kNear];
+    int2 warp[kPlocBlock / 32];
+    int2 before, total;
+};
+
+// Phase 1 of the tile at b0; `carry` counts the merges and survivors of the
+// block's tiles so far. A position's nn entry becomes its partner when it
+// merges, -1 when it stays as it is, -2 when its partner takes it.
+__device__ __forceinline__ void ploc_pair_tile(const float4* cbox, int n, int b0, int* nn, int2* pos, PlocShared& sh,
+                                               int2& carry) {
+    for (int t = threadIdx.x; t < PlocShared::kWindow; t += kPlocBlock) {
+        const int g = b0 - 2 * kPlocRadius + t;
+        const bool in = g >= 0 && g < n;
+        sh.lo[t] = in ? cbox[2 * (long long)g] : make_float4(INFINITY, INFINITY, INFINITY, __int_as_float(-1));
+        sh.hi[t] = in ? cbox[2 * (long long)g + 1] : make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < PlocShared::kNear; t += kPlocBlock) {
+        const int i = b0 - kPlocRadius + t, me = t + kPlocRadius;
+        int bj = -1;
+        if (i >= 0 && i < n) {
+            const float4 lo = sh.lo[me], hi = sh.hi[me];
+            const int s = __float_as_int(lo.w);
+            float best = INFINITY;
+#pragma unroll
+            for (int o = -kPlocRadius; o <= kPlocRadius; o++) {
+                if (o == 0) continue;
+                const float4 l2 = sh.lo[me + o];
+                const float a = merged_area(lo, hi, l2, sh.hi[me + o]);
+                if (__float_as_int(l2.w) == s && a < best) {
+                    best = a;
+                    bj = i + o;
+                }
+            }
+        }
+        sh.near[t] = bj;
+    }
+    __syncthreads();
+    const int i = b0 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j = i < n ? sh.near[threadIdx.x + kPlocRadius] : -1;
+    const bool mutual = j >= 0 && sh.near[j - b0 + kPlocRadius] == i;
+    const bool merges = mutual && i < j, stays = i < n && (!mutual || i < j);
+    const unsigned mm = __ballot_sync(0xffffffffu, merges), ms = __ballot_sync(0xffffffffu, stays);
+    if (lane == 0) sh.warp[warp] = make_int2(__popc(mm), __popc(ms));
+    __syncthreads();
+    int2 at = carry;
+    for (int w = 0; w < kPlocBlock / 32; w++) {
+        const int2 c = sh.warp[w];
+        if (w < warp) {
+            at.x += c.x;
+            at.y += c.y;
+        }
+        carry.x += c.x;
+        carry.y += c.y;
+    }
+    if (i < n) {
+        const unsigned below = (1u << lane) - 1u;
+        nn[i] = merges ? j : stays ? -1 : -2;
+        pos[i] = make_int2(at.x + __popc(mm & below), at.y + __popc(ms & below));
+    }
+    __syncthreads();  // the shared arrays are refilled by the block's next tile
+}
+
 __global__ void __launch_bounds__(kPlocBlock) k_ploc_rounds(PlocRounds a) {
     cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-    __shared__ float4 sLo[kPlocBlock + 2 * kPlocRadius], sHi[kPlocBlock + 2 * kPlocRadius];
-    __shared__ int2 warpSum[kPlocBlock / 32];
-    __shared__ int2 carry;
-    const int per = kPlocBlock * kScanItems;
-    const long long stride = (long long)gridDim.x * blockDim.x;
+    __shared__ PlocShared sh;
     int n = a.N, nodeBase = 0, cur = 0, round = 0;
     bool failed = false;
+    bool alone = false;  // the first block runs the remaining rounds
     while (n > a.nseg) {
         if (round >= a.maxRounds) {
             failed = true;
@@ -1538,30 +1698,61 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_rounds(PlocRounds a) {
         const float4* cbox = cur ? a.cbox[1] : a.cbox[0];
         int* crefOut = cur ? a.cref[0] : a.cref[1];
         float4* cboxOut = cur ? a.cbox[0] : a.cbox[1];
-        for (int b0 = blockIdx.x * kPlocBlock; b0 < n; b0 += gridDim.x * kPlocBlock)
-            ploc_nn_tile(cbox, n, b0, a.nn, sLo, sHi);
-        grid.sync();
-        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-            a.flags[i] = ploc_flag(a.nn, (int)i);
-        grid.sync();
-        const int nb = (n + per - 1) / per;
-        for (int t = blockIdx.x; t < nb; t += gridDim.x) scan2_tile(a.flags, n, t, a.pos, a.sums, warpSum);
-        grid.sync();
-        if (blockIdx.x == 0) scan2_sums_block(a.sums, nb, a.total, warpSum, carry);
-        grid.sync();
-        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-            const int2 pi = a.pos[i], off = a.sums[i / per];
-            ploc_emit_one(cref, cbox, a.nn, a.flags[i], make_int2(pi.x + off.x, pi.y + off.y), (int)i, nodeBase,
-                          a.nodeCap, a.nodes, crefOut, cboxOut, a.err);
+        const int tiles = (n + kPlocBlock - 1) / kPlocBlock;
+        if (n <= kPlocOneBlock) alone = true;
+        if (alone && blockIdx.x != 0) return;
+        const int t0 = alone ? 0 : (int)((long long)tiles * blockIdx.x / gridDim.x);
+        const int t1 = alone ? tiles : (int)((long long)tiles * (blockIdx.x + 1) / gridDim.x);
+        int2 carry = make_int2(0, 0);
+        for (int t = t0; t < t1; t++) ploc_pair_tile(cbox, n, t * kPlocBlock, a.nn, a.pos, sh, carry);
+        int2 base = make_int2(0, 0), total = carry;
+        if (!alone) {
+            if (threadIdx.x == 0) a.sums[blockIdx.x] = carry;
+            grid.sync();
+            int2 lower = make_int2(0, 0), all = make_int2(0, 0);
+            for (int k = threadIdx.x; k < (int)gridDim.x; k += kPlocBlock) {
+                const int2 c = __ldcg(&a.sums[k]);
+                all.x += c.x;
+                all.y += c.y;
+                if (k < (int)blockIdx.x) {
+                    lower.x += c.x;
+                    lower.y += c.y;
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                lower.x += __shfl_xor_sync(0xffffffffu, lower.x, o);
+                lower.y += __shfl_xor_sync(0xffffffffu, lower.y, o);
+                all.x += __shfl_xor_sync(0xffffffffu, all.x, o);
+                all.y += __shfl_xor_sync(0xffffffffu, all.y, o);
+            }
+            if (threadIdx.x == 0) sh.before = sh.total = make_int2(0, 0);
+            __syncthreads();
+            if ((threadIdx.x & 31) == 0) {
+                atomicAdd(&sh.before.x, lower.x);
+                atomicAdd(&sh.before.y, lower.y);
+                atomicAdd(&sh.total.x, all.x);
+                atomicAdd(&sh.total.y, all.y);
+            }
+            __syncthreads();
+            base = sh.before;
+            total = sh.total;
         }
-        grid.sync();
-        const int2 t = *a.total;  // written by block 0 before the last two barriers
-        if (t.x == 0) {
+        for (int t = t0; t < t1; t++) {
+            const int i = t * kPlocBlock + threadIdx.x;
+            if (i >= n) continue;
+            const int j = a.nn[i];
+            const int2 at = a.pos[i];
+            ploc_emit_one(cref, cbox, a.nn, make_int2(j >= 0 ? 1 : 0, j >= -1 ? 1 : 0), make_int2(base.x + at.x, base.y + at.y),
+                          i, nodeBase, a.nodeCap, a.nodes, crefOut, cboxOut, a.err);
+        }
+        if (alone) __syncthreads();
+        else grid.sync();
+        if (total.x == 0) {
             failed = true;
             break;
         }
-        nodeBase += t.x;
-        n = t.y;
+        nodeBase += total.x;
+        n = total.y;
         cur = 1 - cur;
         round++;
     }
@@ -1580,14 +1771,24 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_rounds(PlocRounds a) {
 struct ClusterTree {
     float4* nodes = nullptr;
     std::vector<int> roots;
+    const int* deviceRoots = nullptr;  // in the nodes' allocation
 };
+
+// The box of each scene's root: its two children's.
+__global__ void k_root_boxes(const float4* __restrict__ nodes, const int* __restrict__ roots, int nseg,
+                             mc_aabb* __restrict__ boxes) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nseg) return;
+    boxes[s] = to_aabb(merge_box(load_child_box(nodes, roots[s], 0), load_child_box(nodes, roots[s], 1)));
+}
 
 static mc_status build_ploc(mc_context* ctx, const mc_bvh* bvh, const Seg* dSeg, int nseg, const int32_t* order,
                             const mc_aabb* bounds, ClusterTree& tree, bool coop) {
     const int N = bvh->n, NI = bvh->ni;
     if (NI <= 0 || N < 2) return MC_ERR_UNSUPPORTED;
     const int per = kPlocBlock * kScanItems;
-    const long long nbMax = (N + per - 1) / per;
+    // tile sums of the per-phase launches, block sums of the cooperative one
+    const long long nbMax = std::max<long long>((N + per - 1) / per, 32ll * ctx->sm_count);
     const size_t bytes = (size_t)NI * 64 + 2 * (size_t)N * 4 + 4 * (size_t)N * 16 + (size_t)N * 4 + 2 * (size_t)N * 8 +
                          (size_t)(nbMax + 1) * 8 + 32 + 16 * 16;  // + the 16-byte rounding of each part
     char* mem = nullptr;
@@ -1624,7 +1825,7 @@ static mc_status build_ploc(mc_context* ctx, const mc_bvh* bvh, const Seg* dSeg,
         PlocRounds pr;
         pr.cref[0] = cref[0]; pr.cref[1] = cref[1];
         pr.cbox[0] = cbox[0]; pr.cbox[1] = cbox[1];
-        pr.nn = nn; pr.flags = flags; pr.pos = pos; pr.sums = sums; pr.total = total; pr.state = state;
+        pr.nn = nn; pr.pos = pos; pr.sums = sums; pr.state = state;
         pr.nodes = tree.nodes;
         pr.nodeCap = NI; pr.nseg = nseg; pr.N = N; pr.maxRounds = 4096;
         pr.err = ctx->d_error;
@@ -1684,6 +1885,7 @@ static mc_status build_ploc(mc_context* ctx, const mc_bvh* bvh, const Seg* dSeg,
     if (nodeBase != NI || n != nseg) return fail(set_error(MC_ERR_INVALID, "mc_bvh_build: clustering left %d clusters", n));
     for (int r : tree.roots)
         if (r < 0) return fail(MC_ERR_UNSUPPORTED);  // a scene of one primitive: keep the LBVH
+    tree.deviceRoots = cref[cur];
     // the node block starts the allocation, so freeing it frees everything
     return MC_OK;
 }
@@ -1713,7 +1915,7 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
     if (NI > 0) {
         // surface-area-greedy collapse, level by level from the scene roots
         int* front[2] = {nullptr, nullptr};
-        int* cnt = nullptr;  // [0]: next frontier size; [4..7]: the cooperative collapse's results
+        int* cnt = nullptr;  // [0]: next frontier size; [4..8]: the cooperative collapse's results; [16..]: its block totals
         int4* internal = nullptr;  // per frontier node: its internal slots
         int* blockTotals = nullptr;
         auto release = [&]() {
@@ -1725,7 +1927,7 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
         };
         if (!palloc(ctx, &rootOf, (size_t)NI * sizeof(int)) ||
             !palloc(ctx, &front[0], (size_t)NI * sizeof(int)) ||
-            !palloc(ctx, &front[1], (size_t)NI * sizeof(int)) || !palloc(ctx, &cnt, 8 * sizeof(int)) ||
+            !palloc(ctx, &front[1], (size_t)NI * sizeof(int)) || !palloc(ctx, &cnt, (size_t)(16 + 32 * ctx->sm_count) * sizeof(int)) ||
             !palloc(ctx, &internal, (size_t)NI * sizeof(int4)) ||
             !palloc(ctx, &blockTotals, (size_t)(grid_for(NI, kBlock) + 1) * sizeof(int))) {
             cudaGetLastError();
@@ -1753,8 +1955,8 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
             wl.wideId = wideId;
             wl.rootOf = rootOf;
             wl.internal = internal;
-            wl.blockTotals = blockTotals;
-            wl.total = cnt;
+            wl.tileFirst = blockTotals;
+            wl.blockTotals = cnt + 16;
             wl.out = cnt + 4;
             wl.err = ctx->d_error;
             void* args[] = {&wl};
@@ -1996,27 +2198,39 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
         k_karras<<<grid_for(NI, kBlock), kBlock, 0, ctx->stream>>>(bvh->codes, dSeg, nseg, NI, (float4*)bvh->nodes,
                                                                   bvh->parents, bvh->ref_internal, bvh->ref_leaves,
                                                                   (int2*)ctx->scratch[1].ptr);
-    k_leaves_refit<<<grid_for(N, kBlock), kBlock, 0, ctx->stream>>>(order, boundsRef, N, NI, dSeg, nseg, (float4*)bvh->nodes,
-                                                                   (float4*)bvh->prims, bvh->parents, counters, bvh->ids,
-                                                                   bvh->types, bvh->ref_internal, bvh->ref_leaves,
-                                                                   dRootBoxes, ctx->d_error);
-    if (N == 1) k_single_root<<<1, 1, 0, ctx->stream>>>((float4*)bvh->nodes, boundsRef);
-    if (cudaGetLastError() != cudaSuccess) return fail(set_error(MC_ERR_CUDA, "mc_bvh_build: launch failed"));
-    int flags = 0;
+    // The LBVH's boxes are what the binary layout, the exported reference nodes
+    // and a collapse of the LBVH read; a clustered tree needs its topology alone
+    // (leaf ranks), and its own root box is the scene's: at 1M triangles the
+    // refit is 200 us of a build.
+    const bool wide = o.layout == MC_BVH_LAYOUT_WIDE4 || o.layout == MC_BVH_LAYOUT_WIDE4Q;
+    const bool clusteredOnly = wide && o.builder == MC_BVH_BUILDER_CLUSTERED && !o.keep_reference_nodes && N > 1;
     bvh->seg_bounds.resize(nseg);
-    if (cudaMemcpyAsync(bvh->seg_bounds.data(), dRootBoxes, (size_t)nseg * sizeof(mc_aabb), cudaMemcpyDeviceToHost,
-                        ctx->stream) != cudaSuccess)
-        return fail(cuda_error(cudaGetLastError(), "mc_bvh_build", __FILE__, __LINE__));
-    if ((st = flags_now(ctx, &flags)) != MC_OK) return fail(st);
-    if (flags) return fail(status_from_device_flags(flags));
-    bvh->bounds = bvh->seg_bounds[0];
+    auto leaves = [&](bool boxes) -> mc_status {
+        k_leaves_refit<<<grid_for(N, kBlock), kBlock, 0, ctx->stream>>>(order, boundsRef, N, NI, dSeg, nseg, (float4*)bvh->nodes,
+                                                                       (float4*)bvh->prims, bvh->parents, counters, bvh->ids,
+                                                                       bvh->types, bvh->ref_internal, bvh->ref_leaves,
+                                                                       dRootBoxes, ctx->d_error, boxes);
+        if (N == 1) k_single_root<<<1, 1, 0, ctx->stream>>>((float4*)bvh->nodes, boundsRef);
+        if (cudaGetLastError() != cudaSuccess) return set_error(MC_ERR_CUDA, "mc_bvh_build: launch failed");
+        return MC_OK;
+    };
+    auto root_boxes = [&]() -> mc_status {
+        int f = 0;
+        if (cudaMemcpyAsync(bvh->seg_bounds.data(), dRootBoxes, (size_t)nseg * sizeof(mc_aabb), cudaMemcpyDeviceToHost,
+                            ctx->stream) != cudaSuccess)
+            return cuda_error(cudaGetLastError(), "mc_bvh_build", __FILE__, __LINE__);
+        mc_status s = flags_now(ctx, &f);
+        return s != MC_OK ? s : f ? status_from_device_flags(f) : MC_OK;
+    };
+    if ((st = leaves(!clusteredOnly)) != MC_OK) return fail(st);
+    if (!clusteredOnly && (st = root_boxes()) != MC_OK) return fail(st);
     bvh->seg_prim_off.resize(nseg);
     bvh->bin_roots.resize(nseg);
     for (int s = 0; s < nseg; s++) {
         bvh->seg_prim_off[s] = segs[s].primOff;
         bvh->bin_roots[s] = segs[s].intOff;
     }
-    if (o.layout == MC_BVH_LAYOUT_WIDE4 || o.layout == MC_BVH_LAYOUT_WIDE4Q) {
+    if (wide) {
         const bool coop = o.phase_launches == 0;
         // the wide layouts traverse the collapse of the clustered tree, or of
         // the LBVH when clustering does not apply (a one-primitive scene, a
@@ -2025,6 +2239,13 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
         if (o.builder == MC_BVH_BUILDER_CLUSTERED) {
             ClusterTree tree;
             st = build_ploc(ctx, bvh, dSeg, nseg, order, boundsRef, tree, coop);
+            if (st == MC_OK && clusteredOnly) {
+                k_root_boxes<<<grid_for(nseg, kBlock), kBlock, 0, ctx->stream>>>(tree.nodes, tree.deviceRoots, nseg, dRootBoxes);
+                if ((st = root_boxes()) != MC_OK) {
+                    pool_free(ctx, tree.nodes);
+                    return fail(st);
+                }
+            }
             if (st == MC_OK) {
                 st = build_wide(ctx, bvh, dSeg, nseg, dWideRoot, coop, tree.nodes, &tree.roots);
                 pool_free(ctx, tree.nodes);
@@ -2036,10 +2257,18 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
             if (bvh->wide_nodes) pool_free(ctx, bvh->wide_nodes);
             if (bvh->records) pool_free(ctx, bvh->records);
             bvh->wide_nodes = bvh->records = nullptr;
+            if (clusteredOnly) {
+                if ((st = devbuf_reserve(ctx->scratch[5], (size_t)nodesCount * 4 + 16)) != MC_OK) return fail(st);
+                counters = (int*)ctx->scratch[5].ptr;
+                if (cudaMemsetAsync(counters, 0, (size_t)nodesCount * 4, ctx->stream) != cudaSuccess)
+                    return fail(cuda_error(cudaGetLastError(), "memset", __FILE__, __LINE__));
+                if ((st = leaves(true)) != MC_OK || (st = root_boxes()) != MC_OK) return fail(st);
+            }
             if ((st = build_wide(ctx, bvh, dSeg, nseg, dWideRoot, coop)) != MC_OK) return fail(st);
             bvh->builder = MC_BVH_BUILDER_LBVH;
         }
     }
+    bvh->bounds = bvh->seg_bounds[0];
     if (o.layout == MC_BVH_LAYOUT_WIDE4Q) {
         void* q = nullptr;
         if (!palloc(ctx, &q, (size_t)bvh->wide_count * 64)) {

@@ -1,0 +1,100 @@
+"""Builds at the sizes where the cooperative clustering and collapse change how
+they divide their work (tiles of 256, the rounds one block runs alone, blocks
+with several scenes): the same tree, byte for byte, as the launch-per-phase
+loops, and the same scene bounds and hits as a build that also refits the LBVH."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import mcpt
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = mcpt.Context(0)
+    yield c
+    c.close()
+
+
+def triangles(n, seed):
+    r = np.random.default_rng(seed)
+    v = np.zeros((n, 56), np.float32)
+    c = r.uniform(-1, 1, (n, 1, 3))
+    size = r.choice([0.01, 0.05, 1.5], (n, 1, 1), p=[0.7, 0.29, 0.01])  # a few large ones: many small late rounds
+    v[:, :9] = (c + r.uniform(-1, 1, (n, 3, 3)) * size).reshape(n, 9)
+    return torch.from_numpy(v).cuda()
+
+
+class Scene:
+    def __init__(self, ctx, n, seed):
+        full = triangles(n, seed)
+        self.hot = torch.empty(n * 36, dtype=torch.uint8, device="cuda")
+        self.cold = torch.empty(n * 192, dtype=torch.uint8, device="cuda")
+        self.light = torch.zeros(64, dtype=torch.uint8, device="cuda")
+        mcpt.check(ctx.lib.mc_scene_ingest(ctx.handle, full.data_ptr(), n, None, 0, self.hot.data_ptr(), self.cold.data_ptr(),
+                                           None, None, None))
+        v = mcpt.SceneView()
+        v.tri_hot, v.tri_cold, v.triangle_count, v.lights = self.hot.data_ptr(), self.cold.data_ptr(), n, self.light.data_ptr()
+        self.view, self.n = v, n
+
+
+def hits(ctx, view, bvh, n=2000):
+    r = np.random.default_rng(7)
+    rays = np.zeros((7, n), np.float32)
+    rays[0:3] = r.uniform(-1.2, 1.2, (3, n))
+    d = r.normal(size=(3, n))
+    rays[3:6] = d / np.linalg.norm(d, axis=0)
+    rays = torch.from_numpy(rays).cuda()
+    h = torch.empty(n, 4, dtype=torch.int32, device="cuda")
+    mcpt.check(ctx.lib.mc_trace_closest(ctx.handle, bvh.handle, C.byref(view), rays.data_ptr(), n, 0, h.data_ptr()))
+    return h
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 255, 256, 257, 1023, 1024, 1025, 4099, 75777, 303105])
+@pytest.mark.parametrize("builder", [mcpt.BUILDER_CLUSTERED, mcpt.BUILDER_LBVH])
+def test_single(ctx, n, builder):
+    s = Scene(ctx, n, n)
+    coop = mcpt.Bvh(ctx, s.view, layout=mcpt.LAYOUT_WIDE4, builder=builder)
+    phase = mcpt.Bvh(ctx, s.view, layout=mcpt.LAYOUT_WIDE4, builder=builder, phase_launches=True)
+    refit = mcpt.Bvh(ctx, s.view, layout=mcpt.LAYOUT_WIDE4, builder=builder, keep_reference_nodes=True)
+    binary = mcpt.Bvh(ctx, s.view, layout=mcpt.LAYOUT_BINARY)
+    a, b, c = (x.traversal_arrays() for x in (coop, phase, refit))
+    for x, y, z in zip(a, b, c):
+        assert torch.equal(x, y) and torch.equal(x, z)
+    i = [x.info() for x in (coop, phase, refit, binary)]
+    box = [(q.scene_bounds.lo.x, q.scene_bounds.lo.y, q.scene_bounds.lo.z, q.scene_bounds.hi.x, q.scene_bounds.hi.y,
+            q.scene_bounds.hi.z) for q in i]
+    assert box[0] == box[1] == box[2] == box[3]
+    want = hits(ctx, s.view, binary)
+    for x in (coop, phase, refit):
+        assert torch.equal(hits(ctx, s.view, x), want)
+        x.close()
+    binary.close()
+
+
+@pytest.mark.parametrize("sizes", [(2, 2), (300, 2, 5, 1021, 7), tuple([40] * 60), (2000, 3, 90000, 511)])
+def test_batch(ctx, sizes):
+    scenes = [Scene(ctx, n, 100 + k) for k, n in enumerate(sizes)]
+    views = [s.view for s in scenes]
+    a = mcpt.BatchBvh(ctx, views)
+    b = mcpt.BatchBvh(ctx, views, phase_launches=True)
+    for x, y in zip(mcpt.traversal_arrays(ctx.lib, a.handle), mcpt.traversal_arrays(ctx.lib, b.handle)):
+        assert torch.equal(x, y)
+    a.close()
+    b.close()
+
+
+def test_morton_bounds_over_mixed_blocks(ctx):
+    """Scene bounds of blocks that hold one scene, and their Morton codes."""
+    s = Scene(ctx, 70001, 3)
+    codes = torch.empty(s.n, dtype=torch.int32, device="cuda")
+    box = mcpt.AABB()
+    mcpt.check(ctx.lib.mc_morton_codes(ctx.handle, C.byref(s.view), codes.data_ptr(), C.byref(box)))
+    v = s.hot.view(torch.float32).reshape(-1, 3)
+    eps = torch.tensor(1e-3, device="cuda")
+    assert [box.lo.x, box.lo.y, box.lo.z] == (v.min(0).values - eps).tolist()
+    assert [box.hi.x, box.hi.y, box.hi.z] == (v.max(0).values + eps).tolist()
