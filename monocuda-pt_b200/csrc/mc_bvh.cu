@@ -1587,7 +1587,7 @@ __global__ void k_ploc_advance(const int2* __restrict__ total, int* __restrict__
 }
 
 // Every clustering round in one cooperative launch. The positions of a round
-// are cut into tiles of kPlocBlock, each block takes a contiguous range of
+// are cut into tiles of kPlocTile, each block takes a contiguous range of
 // tiles, and a round is two phases with a grid-wide barrier after each:
 //   1. nearest neighbours of the tile and of kPlocRadius positions on either
 //      side (so that whether a pair is mutual is known without asking another
@@ -1603,7 +1603,8 @@ __global__ void k_ploc_advance(const int2* __restrict__ total, int* __restrict__
 // when every scene is one cluster, after maxRounds rounds (error), or when a
 // round merges nothing (error: the globally closest pair is always mutual);
 // every block computes the same totals, so all run the same rounds and barriers.
-constexpr int kPlocOneBlock = 4 * kPlocBlock;
+constexpr int kPlocTile = kPlocBlock - 2 * kPlocRadius;  // a neighbour search per thread covers the tile and both sides
+constexpr int kPlocOneBlock = 4 * kPlocTile;
 struct PlocRounds {
     int* cref[2];
     float4* cbox[2];
@@ -1617,10 +1618,9 @@ struct PlocRounds {
 };
 
 struct PlocShared {
-    static constexpr int kWindow = kPlocBlock + 4 * kPlocRadius;
-    static constexpr int kNear = kPlocBlock + 2 * kPlocRadius;
+    static constexpr int kWindow = kPlocTile + 4 * kPlocRadius;
     float4 lo[kWindow], hi[kWindow];
-    int near[kNear];
+    int near[kPlocBlock];
     int2 warp[kPlocBlock / 32];
     int2 before, total;
 };
@@ -1637,7 +1637,8 @@ __device__ __forceinline__ void ploc_pair_tile(const float4* cbox, int n, int b0
         sh.hi[t] = in ? cbox[2 * (long long)g + 1] : make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < PlocShared::kNear; t += kPlocBlock) {
+    {
+        const int t = threadIdx.x;
         const int i = b0 - kPlocRadius + t, me = t + kPlocRadius;
         int bj = -1;
         if (i >= 0 && i < n) {
@@ -1659,9 +1660,10 @@ __device__ __forceinline__ void ploc_pair_tile(const float4* cbox, int n, int b0
     }
     __syncthreads();
     const int i = b0 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int j = i < n ? sh.near[threadIdx.x + kPlocRadius] : -1;
+    const bool mine = threadIdx.x < kPlocTile && i < n;
+    const int j = mine ? sh.near[threadIdx.x + kPlocRadius] : -1;
     const bool mutual = j >= 0 && sh.near[j - b0 + kPlocRadius] == i;
-    const bool merges = mutual && i < j, stays = i < n && (!mutual || i < j);
+    const bool merges = mutual && i < j, stays = mine && (!mutual || i < j);
     const unsigned mm = __ballot_sync(0xffffffffu, merges), ms = __ballot_sync(0xffffffffu, stays);
     if (lane == 0) sh.warp[warp] = make_int2(__popc(mm), __popc(ms));
     __syncthreads();
@@ -1675,7 +1677,7 @@ __device__ __forceinline__ void ploc_pair_tile(const float4* cbox, int n, int b0
         carry.x += c.x;
         carry.y += c.y;
     }
-    if (i < n) {
+    if (mine) {
         const unsigned below = (1u << lane) - 1u;
         nn[i] = merges ? j : stays ? -1 : -2;
         pos[i] = make_int2(at.x + __popc(mm & below), at.y + __popc(ms & below));
@@ -1698,13 +1700,13 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_rounds(PlocRounds a) {
         const float4* cbox = cur ? a.cbox[1] : a.cbox[0];
         int* crefOut = cur ? a.cref[0] : a.cref[1];
         float4* cboxOut = cur ? a.cbox[0] : a.cbox[1];
-        const int tiles = (n + kPlocBlock - 1) / kPlocBlock;
+        const int tiles = (n + kPlocTile - 1) / kPlocTile;
         if (n <= kPlocOneBlock) alone = true;
         if (alone && blockIdx.x != 0) return;
         const int t0 = alone ? 0 : (int)((long long)tiles * blockIdx.x / gridDim.x);
         const int t1 = alone ? tiles : (int)((long long)tiles * (blockIdx.x + 1) / gridDim.x);
         int2 carry = make_int2(0, 0);
-        for (int t = t0; t < t1; t++) ploc_pair_tile(cbox, n, t * kPlocBlock, a.nn, a.pos, sh, carry);
+        for (int t = t0; t < t1; t++) ploc_pair_tile(cbox, n, t * kPlocTile, a.nn, a.pos, sh, carry);
         int2 base = make_int2(0, 0), total = carry;
         if (!alone) {
             if (threadIdx.x == 0) a.sums[blockIdx.x] = carry;
@@ -1738,8 +1740,8 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_rounds(PlocRounds a) {
             total = sh.total;
         }
         for (int t = t0; t < t1; t++) {
-            const int i = t * kPlocBlock + threadIdx.x;
-            if (i >= n) continue;
+            const int i = t * kPlocTile + threadIdx.x;
+            if (threadIdx.x >= kPlocTile || i >= n) continue;
             const int j = a.nn[i];
             const int2 at = a.pos[i];
             ploc_emit_one(cref, cbox, a.nn, make_int2(j >= 0 ? 1 : 0, j >= -1 ? 1 : 0), make_int2(base.x + at.x, base.y + at.y),
