@@ -680,12 +680,28 @@ __global__ void k_guide_prepare(const float* master, bf16* blob) {
     }
 }
 
-__global__ void k_guide_reduce(const float* partials, int parts, float* out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int c = 0; c < parts; c++) s += partials[(size_t)c * kParams + i];
-        out[i] = s;
+// Sum of partials[c][i] for c = cBegin .. cEnd - 1, added in that order. Each
+// partial lies a whole parameter vector further on, so the sum waits on memory
+// unless many reads are in flight: sixteen at a time.
+__device__ __forceinline__ float sum_partials(const float* partials, int i, int cBegin, int cEnd) {
+    constexpr int kInFlight = 16;
+    const float* p = partials + (size_t)cBegin * kParams + i;
+    float s = 0.f;
+    int c = cBegin;
+    for (; c + kInFlight <= cEnd; c += kInFlight, p += (size_t)kInFlight * kParams) {
+        float v[kInFlight];
+#pragma unroll
+        for (int k = 0; k < kInFlight; k++) v[k] = p[(size_t)k * kParams];
+#pragma unroll
+        for (int k = 0; k < kInFlight; k++) s += v[k];
     }
+    for (; c < cEnd; c++, p += kParams) s += *p;
+    return s;
+}
+
+__global__ void k_guide_reduce(const float* partials, int parts, float* out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x)
+        out[i] = sum_partials(partials, i, 0, parts);
 }
 
 // The BF16 operand entries of parameter i (its weight, or its bias's hi / lo
@@ -726,10 +742,7 @@ __global__ void __launch_bounds__(32 * kAdamWarps) k_guide_adam(float* master, f
     const int i = blockIdx.x * 32 + lane;
     const int per = (parts + kAdamWarps - 1) / kAdamWarps;
     const int cBegin = w * per, cEnd = min(parts, cBegin + per);
-    float part = 0.f;
-    if (i < kParams)
-        for (int c = cBegin; c < cEnd; c++) part += partials[(size_t)c * kParams + i];
-    slice[w][lane] = part;
+    slice[w][lane] = i < kParams ? sum_partials(partials, i, cBegin, cEnd) : 0.f;
     __syncthreads();
     if (w != 0 || i >= kParams) return;
     float g = 0.f;
@@ -750,6 +763,7 @@ __global__ void k_guide_weight_scale(const float* records, int n, const int* cou
     __shared__ float part[32];
     const int cnt = count ? max(0, min(min(*count, capacity) - offset, stepCap)) : n;
     float s = 0.f;
+#pragma unroll 16
     for (int i = threadIdx.x; i < cnt; i += blockDim.x) s += records[(size_t)i * MC_GUIDE_RECORD_FLOATS + 9];
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
@@ -1112,7 +1126,7 @@ mc_status mc_guide_gradient(mc_guide* g, const float* d_records, int32_t n, floa
     int grid = 0;
     mc_status st = launch_train(g, ctx->stream, d_records, n, nullptr, 0, 0, 0, nullptr, &grid);
     if (st != MC_OK) return st;
-    k_guide_reduce<<<80, 256, 0, ctx->stream>>>(g->partials, grid, d_grad);
+    k_guide_reduce<<<(kParams + 63) / 64, 64, 0, ctx->stream>>>(g->partials, grid, d_grad);
     MC_CUDA(cudaGetLastError());
     double l = 0.0;
     MC_CUDA(cudaMemcpyAsync(&l, g->loss, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
