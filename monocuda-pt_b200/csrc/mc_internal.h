@@ -128,7 +128,7 @@ struct mc_context {
     int trace_blocks[144] = {};
     int trace_blocks_smem[144] = {};     // shared-memory bytes trace_blocks[k] was measured with
     int trace_smem_attr[144] = {};       // dynamic shared memory the variant has been opted in to
-    int paths_blocks[6] = {};            // k_paths: RNG x layout
+    int paths_blocks[3] = {};            // k_paths, per layout
     int paths_blocks_smem = 0;           // shared-memory bytes they were measured with
     int shade_blocks[3] = {};            // Philox, XORWOW, guided
     bool guide_attrs_set = false;        // the guide kernels' shared-memory opt-in is done

@@ -134,6 +134,7 @@ struct TraceArgs {
     int stackCap;                // traversal stack entries per lane, <= MC_STACK_CAPACITY (0: all)
     int threads;                 // block size asked for: 128 or 256 (0: 256)
     int queueCap;                // entries the extend and shadow queues hold (counts past it are clamped)
+    int handOver;                // extend queues of at most this many rays are left to k_paths (0: none)
     // launches with gridded media (MC_MEDIUM_GRID): per shadow slot, the
     // distance of each medium crossing and, for back faces, the homogeneous
     // factor or the crossed primitive of a grid; rays that crossed a grid are
@@ -308,7 +309,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? MC_TRACE_MIN_BLOCKS 
     const int lane = threadIdx.x & 31;
     const unsigned ltmask = lanemask_lt();
     // a queue that overflowed holds queueCap entries (the producer flagged the overflow)
-    const int extCount = a.extCount ? min(*a.extCount, a.queueCap) : a.extN;
+    int extCount = a.extCount ? min(*a.extCount, a.queueCap) : a.extN;
+    if (extCount <= a.handOver) extCount = 0;
     const int shCount = a.shCount ? min(*a.shCount, a.queueCap) : a.shN;
     const int total = extCount + shCount;
     extern __shared__ int traceStack[];
@@ -437,6 +439,7 @@ struct ShadeArgs {
     int* spath;
     int* shCount;
     int capacity;
+    int handOver;     // as in TraceArgs: the bounce's paths go on in k_paths
     int* err;
     // guided shading: per-path mixtures of this bounce, the guide's share of
     // the one-sample MIS, the training records of the first recSlots diffuse
@@ -850,6 +853,7 @@ template <class Rng, bool GUIDED, bool ALIAS = false>
 __global__ void __launch_bounds__(256, GUIDED ? MC_GUIDED_SHADE_BLOCKS : MC_SHADE_BLOCKS) k_shade(ShadeArgs a) {
     const unsigned ltmask = lanemask_lt();
     const int count = min(*a.count, a.capacity);
+    if (count <= a.handOver) return;
     for (int base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
         int q = base + threadIdx.x;
         ShadeOut out;
@@ -1247,12 +1251,15 @@ __global__ void __launch_bounds__(256) k_ratio_track(ShadeArgs a, RatioArgs v) {
 // wave passes through memory (a shadow ray's contribution and length) is rounded
 // there, so its uses here are written with explicit roundings.
 struct PathsArgs {
-    const int* queue;
-    const int* count;
-    int* work;
+    // The bounce taken over is the first of depthLo .. depthHi - 1 whose queue
+    // holds between one and `few` paths (the wave's launches left that bounce
+    // alone, so the later queues are empty).
+    const int* queue[2];
+    int* counters;       // of bounce d: slot d, or d % kRingSlots in a deep wave
+    int ring;
+    int depthLo, depthHi, few;
     int stackCap;
     int gridMedia;       // the wave's trace launches would be the density-grid variant
-    int depth;           // bounce the queued paths are at
     long long* stats;    // extend and shadow rays per depth
     int* err;
 };
@@ -1331,13 +1338,24 @@ MC_D float shadow_ray(const ShadeArgs& a, const PathsArgs& v, const SceneGPU& S,
     return blocked ? 0.0f : T;
 }
 
-template <class Rng, int LAY>
+template <int LAY>
 __global__ void __launch_bounds__(kPathsThreads) k_paths(ShadeArgs a, PathsArgs v) {
+    typedef PhiloxRng Rng;
     extern __shared__ int traceStack[];
     const SharedStack<kPathsThreads> stack(traceStack, v.stackCap);
     const int lane = threadIdx.x & 31;
     const unsigned ltmask = lanemask_lt();
-    const int total = min(*v.count, a.capacity);
+    int first = -1;
+    for (int d0 = v.depthLo; d0 < v.depthHi && first < 0; d0 += 32) {
+        const int d = d0 + lane;
+        const int c = d < v.depthHi ? v.counters[(v.ring ? d % v.ring : d) * MC_COUNTERS_PER_DEPTH] : 0;
+        const unsigned m = __ballot_sync(kFull, c > 0 && c <= v.few);
+        if (m) first = d0 + __ffs(m) - 1;
+    }
+    if (first < 0) return;
+    int* counters = v.counters + (v.ring ? first % v.ring : first) * MC_COUNTERS_PER_DEPTH;
+    const int* queue = v.queue[first & 1];
+    const int total = min(counters[0], a.capacity);
     const int warps = gridDim.x * (kPathsThreads / 32);
     const int width = min(32, (total + warps - 1) / warps);
     bool exhausted = total == 0;
@@ -1348,12 +1366,12 @@ __global__ void __launch_bounds__(kPathsThreads) k_paths(ShadeArgs a, PathsArgs 
         if (!exhausted && take > 0) {
             const int leader = __ffs(idle) - 1;
             int base = 0;
-            if (lane == leader) base = atomicAdd(v.work, take);
+            if (lane == leader) base = atomicAdd(counters + 3, take);
             base = __shfl_sync(kFull, base, leader);
             const int nth = __popc(idle & ltmask);
             if (p < 0 && nth < take && base + nth < total) {
-                p = v.queue[base + nth];
-                depth = v.depth;
+                p = queue[base + nth];
+                depth = first;
             }
             if (base + take >= total) exhausted = true;
         }
@@ -1369,7 +1387,7 @@ __global__ void __launch_bounds__(kPathsThreads) k_paths(ShadeArgs a, PathsArgs 
             ts.root = S.root;
             const int bucket = min(depth, MC_MAX_DEPTH_STATS - 1);
             // the first bounce's extend rays are in the wave's counters already
-            if (depth != v.depth) atomicAdd((unsigned long long*)&v.stats[bucket], 1ull);
+            if (depth != first) atomicAdd((unsigned long long*)&v.stats[bucket], 1ull);
             {
                 TravState s;
                 trav_begin(s, stack, V3(a.ox[p], a.oy[p], a.oz[p]), V3(a.dx[p], a.dy[p], a.dz[p]), a.time[p], 1e30f, ts.root);
@@ -1681,15 +1699,19 @@ static void set_single_scene(TraceArgs& t, const mc_bvh* bvh, int root, const mc
 // cloud 65,800 / 15,100, 960k 26,100 (handed over at 65,536) / 20,700.
 constexpr int kPathsInFlight = 1 << 16;
 constexpr int kPathsInFlightGrid = 1 << 20;
+// Larger waves leave a bounce with at most this many paths, and all after it,
+// to k_paths (4K to 32K measured alike, 64K slower where the paths are long):
+// 600x600 spheres of depth 20 2.81 -> 2.66 ms, 131,044 paths 939 -> 739 us,
+// Cornell boxes 493 -> 423 us, 16 small scenes 2.16 -> 2.12 ms.
+constexpr int kHandOver = 1 << 14;
 
-static void launch_paths(mc_context* ctx, cudaStream_t stream, const ShadeArgs& a, PathsArgs v, int layout, bool philox) {
+static void launch_paths(mc_context* ctx, cudaStream_t stream, const ShadeArgs& a, PathsArgs v, int layout) {
     typedef void (*Kernel)(ShadeArgs, PathsArgs);
-    static const Kernel table[2][3] = {{k_paths<PhiloxRng, 0>, k_paths<PhiloxRng, 1>, k_paths<PhiloxRng, 2>},
-                                       {k_paths<XorwowRng, 0>, k_paths<XorwowRng, 1>, k_paths<XorwowRng, 2>}};
-    const Kernel fn = table[philox ? 0 : 1][layout];
+    static const Kernel table[3] = {k_paths<0>, k_paths<1>, k_paths<2>};
+    const Kernel fn = table[layout];
     if (v.stackCap <= 0 || v.stackCap > MC_STACK_CAPACITY) v.stackCap = MC_STACK_CAPACITY;
     const int smem = kPathsThreads * v.stackCap * (int)sizeof(int);  // at most 32 KB: no opt-in
-    int& blocks = ctx->paths_blocks[(philox ? 0 : 3) + layout];
+    int& blocks = ctx->paths_blocks[layout];
     if (!blocks || ctx->paths_blocks_smem != smem) {
         if (ctx->paths_blocks_smem != smem)
             for (int& b : ctx->paths_blocks) b = 0;
@@ -1890,23 +1912,32 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
     if (guide && train && guidedDepth > 0) guidedDepth = std::max(guidedDepth, guide->cfg.train_vertices + 1);
     // launches of k_paths: not where a variant of the wave's own kernels was
     // asked for (instruments, the watertight test, alias sampling, a queue
-    // limit, the plain mode)
-    const bool pathsOk = !guide && !timeTrace && !countVisits && !alias && isect == MC_ISECT_REFERENCE && persistent &&
+    // limit, the plain mode, the reference's per-pixel generators)
+    const bool pathsOk = philox && !timeTrace && !countVisits && !alias && isect == MC_ISECT_REFERENCE && persistent &&
                          p0.queue_capacity == 0 && maxD > 0;
     const int fewPaths = grid ? kPathsInFlightGrid : kPathsInFlight;
-    const bool smallWave = pathsOk && capacity <= fewPaths;
-    auto enqueue_paths = [&](int d) {
+    const int handPaths = grid ? kPathsInFlightGrid : kHandOver;
+    const bool smallWave = pathsOk && !guide && capacity <= fewPaths;
+    // the first bounce k_paths may take over: guided bounces shade with the
+    // guide, and a guided wave's second trace keeps the primary vertices'
+    // next-event estimates apart
+    const int handFrom = !guide ? 1 : guidedDepth > 0 ? std::max(guidedDepth, 2) : maxD;
+    const bool handOver = pathsOk && !deep && !smallWave && handFrom < maxD;
+    auto enqueue_paths = [&](int lo, int hi, int few) {
         PathsArgs v;
         std::memset(&v, 0, sizeof(v));
-        v.queue = w.queue[d & 1];
-        v.count = slot(d) + 0;
-        v.work = slot(d) + 3;
+        v.queue[0] = w.queue[0];
+        v.queue[1] = w.queue[1];
+        v.counters = C;
+        v.ring = deep ? kRingSlots : 0;
+        v.depthLo = lo;
+        v.depthHi = hi;
+        v.few = few;
         v.stackCap = ta.stackCap;
         v.gridMedia = grid ? 1 : 0;
-        v.depth = d;
         v.stats = ctx->d_stats;
         v.err = ctx->d_error;
-        launch_paths(ctx, stream, sa, v, layout, philox);
+        launch_paths(ctx, stream, sa, v, layout);
         launches++;
     };
     auto enqueue_wave = [&]() -> mc_status {
@@ -1922,7 +1953,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
         int dLast = maxD;    // the last bounce with launches of its own
         bool stop = false, few = false;  // few: the remaining paths go to k_paths
         if (smallWave) {
-            enqueue_paths(0);
+            enqueue_paths(0, 1, capacity);
             dLast = 0;
             dEnd = 1;
         }
@@ -1940,6 +1971,8 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
             if (d > 0) t.shCount = slot(d - 1) + 1;
             else { t.shCount = nullptr; t.shN = 0; }
             t.work = slot(d) + 2;
+            const int leave = handOver && d >= handFrom ? handPaths : 0;  // queues up to this size are left to k_paths
+            t.handOver = leave;
             if (guide && d == 1) {
                 // the primary vertex's NEE lands apart from the sample so that
                 // its training records see only the light through the sampled direction
@@ -1960,9 +1993,10 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
             if (last) {
                 dLast = dEnd = d;
                 if (few) {
-                    enqueue_paths(d);
+                    enqueue_paths(d, d + 1, capacity);
                     dEnd = d + 1;
                 }
+                if (handOver) enqueue_paths(handFrom, maxD, handPaths);
                 break;
             }
             // bounces past the guided depth shade with the cosine lobe alone: no inference
@@ -1990,6 +2024,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
             sd.nextQueue = w.queue[(d + 1) & 1];
             sd.nextCount = slot(d + 1) + 0;
             sd.shCount = slot(d) + 1;
+            sd.handOver = leave;
             if (guidedBounce) {
                 sd.mix = guide->mixtures;
                 sd.guideFrac = guide->cfg.guide_fraction;
@@ -2073,7 +2108,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
                                       (unsigned long long)maxD,
                                       (unsigned long long)((layout << 6) | (medium ? 2 : 0) | (philox ? 4 : 0) |
                                                            (persistent ? 8 : 0) | (n > 1 ? 16 : 0) |
-                                                           (sameScene ? 32 : 0) | (grid ? 1024 : 0) | (smallWave ? 2048 : 0)),
+                                                           (sameScene ? 32 : 0) | (grid ? 1024 : 0) | (smallWave ? 2048 : 0) | (handOver ? 4096 : 0)),
                                       (unsigned long long)isect,
                                       (unsigned long long)ta.refill,
                                       (unsigned long long)(uintptr_t)ta.ts0.nodes,
@@ -2148,7 +2183,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
         MC_CUDA(cudaEventRecord((cudaEvent_t)ctx->table_events[slot], stream));
         if (useGraph) {
             MC_CUDA(cudaGraphLaunch(exec, stream));
-            perWave = smallWave ? 4 : 3 + 2 * maxD + (grid ? maxD : 0);
+            perWave = smallWave ? 4 : 3 + 2 * maxD + (grid ? maxD : 0) + (handOver ? 1 : 0);
         } else {
             if ((st = enqueue_wave()) != MC_OK) return st;
         }

@@ -76,6 +76,7 @@ def same(ctx, dev, bvh, cam, *a, **kw):
     (127, 33, 3, 20, mcpt.LAYOUT_BINARY, mcpt.RNG_PHILOX, False),
     (128, 128, 4, 64, mcpt.LAYOUT_WIDE4Q, mcpt.RNG_PHILOX, True),   # exactly the largest one-launch wave
     (128, 129, 4, 6, mcpt.LAYOUT_WIDE4, mcpt.RNG_PHILOX, False),    # just above it
+    (300, 301, 1, 40, mcpt.LAYOUT_WIDE4, mcpt.RNG_PHILOX, True),    # hands its last bounces over
     (90, 70, 2, 12, mcpt.LAYOUT_WIDE4, mcpt.RNG_XORWOW, True),
     (90, 70, 2, 1, mcpt.LAYOUT_WIDE4, mcpt.RNG_PHILOX, True)])
 def test_mixed_materials(ctx, w, h, spp, depth, layout, rng, sky):
