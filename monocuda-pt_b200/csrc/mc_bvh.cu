@@ -806,9 +806,10 @@ __global__ void __launch_bounds__(kBlock) k_wide_level_write(const int4* __restr
 // contiguous range of a level's tiles: it counts its internal slots, and after a
 // grid-wide barrier adds up the totals of the blocks before it and writes; a
 // second barrier ends the level. Ids follow the frontier's order, as with the
-// per-level launches. Levels of up to kWideOneBlock nodes (the first ones, and
-// the last) run in the first block without grid-wide barriers. Every block reads
-// the same totals, so all run the same levels. With three barriers on every
+// per-level launches. Runs of levels of up to kWideOneBlock nodes (the first ones,
+// the last, and where a frontier shrinks on the way) are the first block's, with
+// one grid-wide barrier after the run: a frontier can grow again, so every block
+// stays to the end. All read the same totals, so all run the same levels. With three barriers on every
 // level 1M triangles took 370 us. Ends when a level adds no internal node, after
 // maxLevels + 1 levels, or when the wide ids would pass the node count (error).
 constexpr int kWideOneBlock = 4 * kBlock;
@@ -864,26 +865,24 @@ __global__ void __launch_bounds__(kBlock) k_wide_levels(WideLevels a) {
         __syncthreads();
         advance(m);
     };
-    if (blockIdx.x == 0) {
-        while (n > 0 && n <= kWideOneBlock && levels <= a.maxLevels && !bad) level_alone();
-        if (threadIdx.x == 0) {
-            a.out[0] = levels;
-            a.out[1] = idBase;
-            a.out[2] = n;
-            a.out[3] = bad ? 1 : 0;
-            a.out[4] = cur;
-        }
-    }
-    grid.sync();
-    levels = __ldcg(&a.out[0]);
-    idBase = __ldcg(&a.out[1]);
-    n = __ldcg(&a.out[2]);
-    bad = __ldcg(&a.out[3]) != 0;
-    cur = __ldcg(&a.out[4]);
     while (n > 0 && levels <= a.maxLevels && !bad) {
         if (n <= kWideOneBlock) {
-            if (blockIdx.x != 0) return;
-            level_alone();
+            if (blockIdx.x == 0) {
+                while (n > 0 && n <= kWideOneBlock && levels <= a.maxLevels && !bad) level_alone();
+                if (threadIdx.x == 0) {
+                    a.out[0] = levels;
+                    a.out[1] = idBase;
+                    a.out[2] = n;
+                    a.out[3] = bad ? 1 : 0;
+                    a.out[4] = cur;
+                }
+            }
+            grid.sync();
+            levels = __ldcg(&a.out[0]);
+            idBase = __ldcg(&a.out[1]);
+            n = __ldcg(&a.out[2]);
+            bad = __ldcg(&a.out[3]) != 0;
+            cur = __ldcg(&a.out[4]);
             continue;
         }
         const int tiles = (n + kBlock - 1) / kBlock;

@@ -30,8 +30,8 @@ def triangles(n, seed):
 
 
 class Scene:
-    def __init__(self, ctx, n, seed):
-        full = triangles(n, seed)
+    def __init__(self, ctx, n, seed, full=None):
+        full = triangles(n, seed) if full is None else full
         self.hot = torch.empty(n * 36, dtype=torch.uint8, device="cuda")
         self.cold = torch.empty(n * 192, dtype=torch.uint8, device="cuda")
         self.light = torch.zeros(64, dtype=torch.uint8, device="cuda")
@@ -54,7 +54,7 @@ def hits(ctx, view, bvh, n=2000):
     return h
 
 
-@pytest.mark.parametrize("n", [1, 2, 3, 255, 256, 257, 1023, 1024, 1025, 4099, 75777, 303105])
+@pytest.mark.parametrize("n", [1, 2, 3, 255, 256, 257, 1023, 1024, 1025, 4099, 75777, 303105, 700001])
 @pytest.mark.parametrize("builder", [mcpt.BUILDER_CLUSTERED, mcpt.BUILDER_LBVH])
 def test_single(ctx, n, builder):
     s = Scene(ctx, n, n)
@@ -74,6 +74,43 @@ def test_single(ctx, n, builder):
         assert torch.equal(hits(ctx, s.view, x), want)
         x.close()
     binary.close()
+
+
+def level_sizes(nodes):
+    """Wide nodes per level of a tree, from its 128-byte nodes."""
+    refs = nodes.cpu().numpy().view(np.int32).reshape(-1, 32)[:, 24:28]
+    front, sizes = np.array([0]), []
+    while len(front):
+        sizes.append(len(front))
+        children = refs[front].ravel()
+        front = children[(children >= 0) & (children < len(refs))]
+    return sizes
+
+
+@pytest.mark.parametrize("dense", [30000, 30001])
+def test_frontier_that_grows_again(ctx, dense):
+    """A wide level of many nodes, then a few levels of a chain, then many again:
+    the collapse goes from all blocks to one and back."""
+    r = np.random.default_rng(dense)
+    far, chain = 30000, 27
+    c = np.concatenate([r.uniform(-0.01, 0.01, (dense, 1, 3)), np.zeros((chain, 1, 3)),
+                        r.uniform(-2e6, 2e6, (far, 1, 3)) + [[[2e7, 7e5, 7e5]]]])
+    size = np.concatenate([np.full(dense, 1e-3), 0.02 * 1.5 ** np.arange(chain), np.full(far, 100.0)])[:, None, None]
+    shape = r.uniform(-1, 1, (len(c), 3, 3))
+    shape[dense:dense + chain] = [[-1, -1, -1], [1, -1, 1], [0, 1, 0]]
+    full = np.zeros((len(c), 56), np.float32)
+    full[:, :9] = (c + shape * size).reshape(len(c), 9)
+    s = Scene(ctx, len(c), 0, torch.from_numpy(full).cuda())
+    phase = mcpt.Bvh(ctx, s.view, layout=mcpt.LAYOUT_WIDE4, phase_launches=True)
+    want = phase.traversal_arrays()
+    sizes = level_sizes(want[0])
+    big = [k for k, n in enumerate(sizes) if n > 1024]
+    assert any(n <= 1024 for n in sizes[big[0]:big[-1]]), sizes
+    coop = mcpt.Bvh(ctx, s.view, layout=mcpt.LAYOUT_WIDE4)
+    for x, y in zip(coop.traversal_arrays(), want):
+        assert torch.equal(x, y)
+    coop.close()
+    phase.close()
 
 
 @pytest.mark.parametrize("sizes", [(2, 2), (300, 2, 5, 1021, 7), tuple([40] * 60), (2000, 3, 90000, 511)])
