@@ -612,9 +612,9 @@ MC_API mc_status mc_bvh_get_info(const mc_bvh* bvh, mc_bvh_info* info);
  * (n-1) and leaves (n) as mc_bvh_node. Needs keep_reference_nodes for nodes. */
 MC_API mc_status mc_bvh_export(const mc_bvh* bvh, uint32_t* d_codes, int32_t* d_ids, int32_t* d_types,
                                mc_bvh_node* d_internal, mc_bvh_node* d_leaves);
-/* Copies of the arrays the traversal reads (device buffers, either may be
- * NULL): the node array (mc_bvh_info.node_bytes bytes) and the leaf-ordered
- * primitive records (mc_bvh_info.prim_bytes bytes), e.g. to store a built tree
+/* Copies of a tree's traversal data (device buffers, either may be NULL): the
+ * node array (mc_bvh_info.node_bytes bytes) and the leaf-ordered primitive
+ * records (mc_bvh_info.prim_bytes bytes: vertices, id and type), e.g. to store a built tree
  * or to compare two builds byte for byte. No counterpart in the reference,
  * whose traversal reads its exported node layout directly. */
 MC_API mc_status mc_bvh_export_traversal(const mc_bvh* bvh, void* d_nodes, void* d_prims);

@@ -23,6 +23,10 @@ typedef struct CUstream_st* cudaStream_t;
 // Child reference of an unused slot in a 4-wide node.
 #define MC_WIDE_EMPTY 0x7FFFFFFF
 
+// Traversal form of a launch whose trees all have octant nodes (the public
+// layouts are 0..2).
+#define MC_LAYOUT_OCTANT 3
+
 namespace mc {
 
 // Records the message for mc_last_error() and returns s.
@@ -125,10 +129,10 @@ struct mc_context {
     // launch configurations measured on this context's device (occupancy of a
     // kernel variant, its opt-in shared-memory size), filled on first use; a
     // context is used by one host thread at a time, so these need no lock
-    int trace_blocks[144] = {};
-    int trace_blocks_smem[144] = {};     // shared-memory bytes trace_blocks[k] was measured with
-    int trace_smem_attr[144] = {};       // dynamic shared memory the variant has been opted in to
-    int paths_blocks[3] = {};            // k_paths, per layout
+    int trace_blocks[192] = {};
+    int trace_blocks_smem[192] = {};     // shared-memory bytes trace_blocks[k] was measured with
+    int trace_smem_attr[192] = {};       // dynamic shared memory the variant has been opted in to
+    int paths_blocks[4] = {};            // k_paths, per traversal form
     int paths_blocks_smem = 0;           // shared-memory bytes they were measured with
     int shade_blocks[3] = {};            // Philox, XORWOW, guided
     bool guide_attrs_set = false;        // the guide kernels' shared-memory opt-in is done
@@ -154,6 +158,7 @@ struct mc_bvh {
     void* records = nullptr;           // what the traversal reads: 64-byte primitive records (mc_traverse.cuh) in leaf
                                        // order (binary layout) or in the reference's visit order (wide layouts)
     void* wide_nodes = nullptr;        // 4-wide nodes, 128 B each (layout MC_BVH_LAYOUT_WIDE4)
+    void* octant_nodes = nullptr;      // the same nodes in octant form, 192 B each, or null (large trees, other layouts)
     long long wide_count = 0;
     int wide_levels = -1;              // levels of the greedy 4-wide tree (a ray's stack holds <= 3 per level), -1 unknown
     // reference representation (optional)

@@ -1244,8 +1244,10 @@ __global__ void __launch_bounds__(256) k_ratio_track(ShadeArgs a, RatioArgs v) {
 // arithmetic of the wave's separate launches, so images and random draws are
 // the same. A wave pays a trace and a shade launch per bounce, each as long as
 // its slowest ray; with too few paths to fill the GPU that latency is all there
-// is, and here a path waits for its own rays only: a 64x48 preview 278 -> 164 us,
-// the 333x180 cloud frame of depth 1000 39.1 -> 11.0 ms. Launched where
+// is, and here a path waits for its own rays only: a 64x48 preview 278 -> 164 us
+// (161 with octant nodes),
+// the 333x180 cloud frame of depth 1000 39.1 -> 11.0 ms (8.8 with the trackers'
+// random numbers drawn ahead). Launched where
 // kPathsInFlight says.
 // Lanes per warp as in k_trace: one path per warp when there are few. What the
 // wave passes through memory (a shadow ray's contribution and length) is rounded
@@ -1498,8 +1500,9 @@ typedef void (*TraceKernel)(TraceArgs);
 #define MC_TK(L, B) {MC_TKM(false, L, B), MC_TKM(true, L, B)}
 // medium: 0 none, 1 homogeneous media only, 2 media with density grids
 TraceKernel trace_kernel(bool batch, int layout, bool count, int medium, int isect) {
-    static const TraceKernel table[2][3][2][3][2] = {{MC_TK(0, false), MC_TK(1, false), MC_TK(2, false)},
-                                                     {MC_TK(0, true), MC_TK(1, true), MC_TK(2, true)}};
+    static const TraceKernel table[2][4][2][3][2] = {
+        {MC_TK(0, false), MC_TK(1, false), MC_TK(2, false), MC_TK(3, false)},
+        {MC_TK(0, true), MC_TK(1, true), MC_TK(2, true), MC_TK(3, true)}};
     return table[batch ? 1 : 0][layout][count ? 1 : 0][medium][isect ? 1 : 0];
 }
 // The 128-thread variant, compiled for launches of the reference intersector
@@ -1507,9 +1510,10 @@ TraceKernel trace_kernel(bool batch, int layout, bool count, int medium, int ise
 #define MC_TK128(B)                                                                                     \
     {{k_trace<0, 0, false, 0, B, 128>, k_trace<0, 1, false, 0, B, 128>},                                \
      {k_trace<0, 0, false, 1, B, 128>, k_trace<0, 1, false, 1, B, 128>},                                \
-     {k_trace<0, 0, false, 2, B, 128>, k_trace<0, 1, false, 2, B, 128>}}
+     {k_trace<0, 0, false, 2, B, 128>, k_trace<0, 1, false, 2, B, 128>},                                \
+     {k_trace<0, 0, false, 3, B, 128>, k_trace<0, 1, false, 3, B, 128>}}
 TraceKernel trace_kernel_128(bool batch, int layout, int medium) {
-    static const TraceKernel table[2][3][2] = {MC_TK128(false), MC_TK128(true)};
+    static const TraceKernel table[2][4][2] = {MC_TK128(false), MC_TK128(true)};
     return table[batch ? 1 : 0][layout][medium];
 }
 
@@ -1531,7 +1535,7 @@ void launch_trace(mc_context* ctx, cudaStream_t stream, const TraceArgs& t0, int
     const int smem = threads * t.stackCap * (int)sizeof(int);
     TraceKernel fn = small ? trace_kernel_128(batch, layout, medium) : trace_kernel(batch, layout, count, medium, isect);
     const int key = medium + 3 * (isect ? 1 : 0) + 6 * (count ? 1 : 0) + 12 * (batch ? 1 : 0) + 24 * layout +
-                    72 * (small ? 1 : 0);  // < 144
+                    96 * (small ? 1 : 0);  // < 192
     if (smem > 48 * 1024 && ctx->trace_smem_attr[key] < smem) {
         cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         ctx->trace_smem_attr[key] = smem;
@@ -1646,12 +1650,21 @@ mc_status rng_reset(mc_context* ctx, int pixels, unsigned long long seed) {
     return MC_OK;
 }
 
-static SceneGPU scene_gpu(mc_context* ctx, const mc_bvh* shared, const WaveItem& it, int pathOffset, uint32_t sample) {
+// The node array a launch of the given traversal form reads (form: the tree's
+// layout, or MC_LAYOUT_OCTANT where every tree of the launch has octant nodes).
+static int traversal_form(const mc_bvh* b) { return b->octant_nodes ? MC_LAYOUT_OCTANT : b->layout; }
+static const float4* traversal_nodes(const mc_bvh* b, int form) {
+    return (const float4*)(form == MC_LAYOUT_OCTANT           ? b->octant_nodes
+                           : b->layout == MC_BVH_LAYOUT_BINARY ? b->nodes
+                                                               : b->wide_nodes);
+}
+
+static SceneGPU scene_gpu(mc_context* ctx, const mc_bvh* shared, const WaveItem& it, int pathOffset, uint32_t sample,
+                          int form) {
     SceneGPU g;
     std::memset(&g, 0, sizeof(g));
     const mc_bvh* bvh = it.bvh ? it.bvh : shared;
-    const bool wide = bvh->layout != MC_BVH_LAYOUT_BINARY;
-    g.nodes = (const float4*)(wide ? bvh->wide_nodes : bvh->nodes);
+    g.nodes = traversal_nodes(bvh, form);
     g.prims = (const float4*)bvh->records;
     g.root = it.root;
     g.spheres = it.view->spheres;
@@ -1679,9 +1692,8 @@ static SceneGPU scene_gpu(mc_context* ctx, const mc_bvh* shared, const WaveItem&
 }
 
 // The scene of a single-scene trace launch, passed as kernel parameters.
-static void set_single_scene(TraceArgs& t, const mc_bvh* bvh, int root, const mc_scene_view* v) {
-    const bool wide = bvh->layout != MC_BVH_LAYOUT_BINARY;
-    t.ts0.nodes = (const float4*)(wide ? bvh->wide_nodes : bvh->nodes);
+static void set_single_scene(TraceArgs& t, const mc_bvh* bvh, int root, const mc_scene_view* v, int form) {
+    t.ts0.nodes = traversal_nodes(bvh, form);
     t.ts0.prims = (const float4*)bvh->records;
     t.ts0.root = root;
     t.medium0 = v->has_medium;
@@ -1701,13 +1713,13 @@ constexpr int kPathsInFlight = 1 << 16;
 constexpr int kPathsInFlightGrid = 1 << 20;
 // Larger waves leave a bounce with at most this many paths, and all after it,
 // to k_paths (4K to 32K measured alike, 64K slower where the paths are long):
-// 600x600 spheres of depth 20 2.81 -> 2.66 ms, 131,044 paths 939 -> 739 us,
-// Cornell boxes 493 -> 423 us, 16 small scenes 2.16 -> 2.12 ms.
+// 600x600 spheres of depth 20 2.81 -> 2.66 ms (2.55 with octant nodes), 131,044
+// paths 939 -> 739 us, Cornell boxes 493 -> 423 us, 16 small scenes 2.16 -> 2.12 ms.
 constexpr int kHandOver = 1 << 14;
 
 static void launch_paths(mc_context* ctx, cudaStream_t stream, const ShadeArgs& a, PathsArgs v, int layout) {
     typedef void (*Kernel)(ShadeArgs, PathsArgs);
-    static const Kernel table[3] = {k_paths<0>, k_paths<1>, k_paths<2>};
+    static const Kernel table[4] = {k_paths<0>, k_paths<1>, k_paths<2>, k_paths<3>};
     const Kernel fn = table[layout];
     if (v.stackCap <= 0 || v.stackCap > MC_STACK_CAPACITY) v.stackCap = MC_STACK_CAPACITY;
     const int smem = kPathsThreads * v.stackCap * (int)sizeof(int);  // at most 32 KB: no opt-in
@@ -1740,7 +1752,10 @@ static void default_shape(TraceArgs& t, int levels, int isect) {
 mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, int n, bool useGraph, bool timed,
                     RenderTiming* tm, mc_guide* guide, bool train) {
     const mc_render_params& p0 = *items[0].p;
-    const int layout = bvh->layout;
+    // octant nodes where every tree of the wave has them
+    bool octant = true;
+    for (int i = 0; i < n; i++) octant &= (items[i].bvh ? items[i].bvh : bvh)->octant_nodes != nullptr;
+    const int layout = octant ? MC_LAYOUT_OCTANT : bvh->layout;
     const bool philox = p0.rng == MC_RNG_PHILOX;
     const int isect = p0.intersector;
     const bool persistent = p0.persistent != 0;
@@ -1838,7 +1853,8 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
     if (countVisits) ta.counts = (unsigned long long*)(ctx->d_stats + 2 * MC_MAX_DEPTH_STATS);
     if (sameScene) {
         // one scene: the trace reads it from kernel parameters
-        set_single_scene(ta, items[0].bvh ? items[0].bvh : bvh, items[0].root, items[0].view);
+        set_single_scene(ta, items[0].bvh ? items[0].bvh : bvh, items[0].root, items[0].view,
+                         layout);
         ta.sceneOf = nullptr;
     }
 
@@ -2160,7 +2176,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
             const int r = std::min(m, items[i].p->spp - wv * m);
             waveR = std::max(waveR, r);
             const int px = items[i].p->width * items[i].p->height;
-            SceneGPU g = scene_gpu(ctx, bvh, items[i], off, (uint32_t)(items[i].p->first_sample + wv * m));
+            SceneGPU g = scene_gpu(ctx, bvh, items[i], off, (uint32_t)(items[i].p->first_sample + wv * m), layout);
             g.pathStride = r;
             g.pixelOffset = pix;
             h->scenes[k++] = g;
@@ -2286,7 +2302,8 @@ mc_status render_items(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items
 // The single-scene trace arguments and launch shape of the ray-set entry points.
 static void ray_set_scene(TraceArgs& t, const mc_bvh* bvh, const mc_scene_view* scene, int isect) {
     default_shape(t, shape_levels(bvh), isect);
-    set_single_scene(t, bvh, bvh->layout != MC_BVH_LAYOUT_BINARY ? bvh->wide_roots[0] : bvh->bin_roots[0], scene);
+    set_single_scene(t, bvh, bvh->layout != MC_BVH_LAYOUT_BINARY ? bvh->wide_roots[0] : bvh->bin_roots[0], scene,
+                     traversal_form(bvh));
 }
 
 }  // namespace mc
@@ -2432,7 +2449,7 @@ mc_status mc_trace_closest(mc_context* ctx, const mc_bvh* bvh, const mc_scene_vi
     t.dx = d_rays + 3 * N; t.dy = d_rays + 4 * N; t.dz = d_rays + 5 * N; t.time = d_rays + 6 * N;
     t.hits = d_hits;
     t.work = work;
-    mc::launch_trace(ctx, ctx->stream, t, bvh->layout, false, intersector, !plain, (n + 255) / 256);
+    mc::launch_trace(ctx, ctx->stream, t, mc::traversal_form(bvh), false, intersector, !plain, (n + 255) / 256);
     MC_CUDA(cudaGetLastError());
     int flags = 0;
     MC_CUDA(cudaMemcpyAsync(&flags, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2466,7 +2483,7 @@ mc_status mc_trace_any(mc_context* ctx, const mc_bvh* bvh, const mc_scene_view* 
     t.smax = d_tmax;
     t.occluded = d_occluded;
     t.work = work;
-    mc::launch_trace(ctx, ctx->stream, t, bvh->layout, false, intersector, !plain, (n + 255) / 256);
+    mc::launch_trace(ctx, ctx->stream, t, mc::traversal_form(bvh), false, intersector, !plain, (n + 255) / 256);
     MC_CUDA(cudaGetLastError());
     int flags = 0;
     MC_CUDA(cudaMemcpyAsync(&flags, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));

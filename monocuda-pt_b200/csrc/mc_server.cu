@@ -48,6 +48,9 @@ struct ServerRequest {
     double submit_s = 0, admit_s = 0, done_s = 0;
 };
 
+// What a scene's BVH is charged against the budget: nodes, 96 bytes of leaf data
+// a primitive, codes and order. (The leaf records take 64 of the 96; the octant
+// nodes of a small tree, at most 50 MB, come out of the rest or beside it.)
 long long bvh_bytes(const mc_bvh* b) {
     long long n = b->n;
     long long s = b->node_bytes + n * 48 + b->wide_count * 128 + n * 48 + 3 * n * 4 + (2 * n) * 4;

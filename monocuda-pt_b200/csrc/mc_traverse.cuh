@@ -12,6 +12,7 @@
 // right), internal children are descended left first with the right one
 // pushed. Closest hits keep the first primitive found at equal t (strict <).
 #pragma once
+#include "mc_internal.h"
 #include "mc_math.cuh"
 
 namespace mc {
@@ -48,6 +49,7 @@ struct TravState {
     int hitLeaf;    // leaf slot of the closest hit, -1 none
     int node;
     int sp;         // stack position (SharedStack byte offset)
+    int xy, z;      // octant nodes: where the near planes of this ray's octant sit (float4 index)
 };
 
 template <class Stack>
@@ -61,6 +63,9 @@ MC_D void trav_restart(TravState& s, const Stack& stack, float tmax, int root) {
 template <class Stack>
 MC_D void trav_begin(TravState& s, const Stack& stack, const V3& o, const V3& d, float time, float tmax, int root) {
     s.r = make_ray_inv(o, d);
+    const bool nx = s.r.ix < 0.0f, ny = s.r.iy < 0.0f;
+    s.xy = nx ? (ny ? 2 : 6) : (ny ? 4 : 0);
+    s.z = s.r.iz < 0.0f ? 10 : 8;
     s.time = time;
     trav_restart(s, stack, tmax, root);
 }
@@ -110,8 +115,10 @@ struct TravCount {
 template <bool ANY, int ISECT, bool COUNT, class Stack>
 MC_D int trav_step(const TraceScene& sc, TravState& s, const Stack& stack, const WatertightRay& w, int* err,
                    TravCount* cnt) {
-    const float4* nd = sc.nodes + (long long)s.node * 4;
-    float4 a = ldg4(nd + 0), b = ldg4(nd + 1), c = ldg4(nd + 2), d = ldg4(nd + 3);
+    const float4* nd = sc.nodes + (size_t)((unsigned)s.node * 4u);
+    float4 a, b, c, d;
+    ldg8(nd, a, b);
+    ldg8(nd + 2, c, d);
     int lref = __float_as_int(d.x), rref = __float_as_int(d.y);
     bool oL = hit_box(s.r, a.x, a.y, a.z, a.w, b.x, b.y, s.tmax);
     bool oR = hit_box(s.r, b.z, b.w, c.x, c.y, c.z, c.w, s.tmax);
@@ -195,10 +202,6 @@ MC_D bool slab_hit(float e0, float e1, float e2, float x0, float x1, float x2, f
     return !(fminf(min3(tfar, x0, x1), x2) <= tnear);
 }
 
-MC_D float4 pick(bool c, const float4& a, const float4& b) {
-    return make_float4(c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z, c ? a.w : b.w);
-}
-
 MC_D void cswap(float& ka, int& va, float& kb, int& vb) {
     if (kb < ka) {
         float tk = ka; ka = kb; kb = tk;
@@ -218,36 +221,64 @@ MC_D float q_scale(unsigned exps, int axis) {
     return __int_as_float((e + 127) << 23);
 }
 
-// QUANT: 64-byte quantised nodes with conservative boxes (more boxes pass; the
-// leaf tests and the rank rule decide the hit as with exact boxes).
-template <bool ANY, int ISECT, bool COUNT, class Stack, bool QUANT>
+MC_D float4 pick(bool c, const float4& a, const float4& b) {
+    return make_float4(c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z, c ? a.w : b.w);
+}
+
+// FORM: MC_BVH_LAYOUT_WIDE4 (128-byte nodes, near and far planes by select),
+// MC_LAYOUT_OCTANT (the same nodes in 192 bytes, by address: float4 0..7 the x
+// and y planes as low low, high high, low high, high low; 8..11 low z and high
+// z, each followed by the references) or MC_BVH_LAYOUT_WIDE4Q (64-byte
+// quantised nodes with conservative boxes: more boxes pass, the leaf tests and
+// the rank rule decide the hit as with exact boxes).
+template <bool ANY, int ISECT, bool COUNT, class Stack, int FORM>
 MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, const WatertightRay& w, int* err,
                     TravCount* cnt) {
-    float4 lx, ly, lz, hx, hy, hz, rf;  // low and high planes of the four children, their references
-    if (QUANT) {
+    float4 ax, ay, az, bx, by, bz, rf;  // near and far planes of the four children, their references
+    if (FORM == MC_BVH_LAYOUT_WIDE4Q) {
         const float4* nd = sc.nodes + (size_t)((unsigned)s.node * 4u);
         float4 h, q0, q1;
         ldg8(nd, h, q0);
         ldg8(nd + 2, q1, rf);
         const unsigned ex = (unsigned)__float_as_int(h.w);
         const float sx = q_scale(ex, 0), sy = q_scale(ex, 1), sz = q_scale(ex, 2);
-        lx = q_planes(h.x, sx, (unsigned)__float_as_int(q0.x));
-        ly = q_planes(h.y, sy, (unsigned)__float_as_int(q0.y));
-        lz = q_planes(h.z, sz, (unsigned)__float_as_int(q0.z));
-        hx = q_planes(h.x, sx, (unsigned)__float_as_int(q0.w));
-        hy = q_planes(h.y, sy, (unsigned)__float_as_int(q1.x));
-        hz = q_planes(h.z, sz, (unsigned)__float_as_int(q1.y));
-    } else {
+        const unsigned lx = (unsigned)__float_as_int(q0.x), hx = (unsigned)__float_as_int(q0.w);
+        const unsigned ly = (unsigned)__float_as_int(q0.y), hy = (unsigned)__float_as_int(q1.x);
+        const unsigned lz = (unsigned)__float_as_int(q0.z), hz = (unsigned)__float_as_int(q1.y);
+        const bool nx = s.r.ix < 0.0f, ny = s.r.iy < 0.0f, nz = s.r.iz < 0.0f;
+        ax = q_planes(h.x, sx, nx ? hx : lx);
+        bx = q_planes(h.x, sx, nx ? lx : hx);
+        ay = q_planes(h.y, sy, ny ? hy : ly);
+        by = q_planes(h.y, sy, ny ? ly : hy);
+        az = q_planes(h.z, sz, nz ? hz : lz);
+        bz = q_planes(h.z, sz, nz ? lz : hz);
+    } else if (FORM == MC_BVH_LAYOUT_WIDE4) {
         const float4* nd = sc.nodes + (size_t)((unsigned)s.node * 8u);
+        float4 lx, ly, lz, hx, hy, hz;
         ldg8(nd, lx, ly);
         ldg8(nd + 2, lz, hx);
         ldg8(nd + 4, hy, hz);
         rf = ldg4(nd + 6);
+        const bool nx = s.r.ix < 0.0f, ny = s.r.iy < 0.0f, nz = s.r.iz < 0.0f;
+        ax = pick(nx, hx, lx);
+        bx = pick(nx, lx, hx);
+        ay = pick(ny, hy, ly);
+        by = pick(ny, ly, hy);
+        az = pick(nz, hz, lz);
+        bz = pick(nz, lz, hz);
+    } else {
+        const unsigned nd = (unsigned)s.node * 12u;
+        ldg8(sc.nodes + (nd + (unsigned)s.xy), ax, ay);
+        ldg8(sc.nodes + (nd + ((unsigned)s.xy ^ 2u)), bx, by);
+        ldg8(sc.nodes + (nd + (unsigned)s.z), az, rf);
+        bz = ldg4(sc.nodes + (nd + 18u - (unsigned)s.z));
     }
-    const bool sx = s.r.ix < 0.0f, sy = s.r.iy < 0.0f, sz = s.r.iz < 0.0f;
-    const float4 ax = slab_t4(pick(sx, hx, lx), s.r.o.x, s.r.ix), bx = slab_t4(pick(sx, lx, hx), s.r.o.x, s.r.ix);
-    const float4 ay = slab_t4(pick(sy, hy, ly), s.r.o.y, s.r.iy), by = slab_t4(pick(sy, ly, hy), s.r.o.y, s.r.iy);
-    const float4 az = slab_t4(pick(sz, hz, lz), s.r.o.z, s.r.iz), bz = slab_t4(pick(sz, lz, hz), s.r.o.z, s.r.iz);
+    ax = slab_t4(ax, s.r.o.x, s.r.ix);
+    bx = slab_t4(bx, s.r.o.x, s.r.ix);
+    ay = slab_t4(ay, s.r.o.y, s.r.iy);
+    by = slab_t4(by, s.r.o.y, s.r.iy);
+    az = slab_t4(az, s.r.o.z, s.r.iz);
+    bz = slab_t4(bz, s.r.o.z, s.r.iz);
     const int ref[4] = {__float_as_int(rf.x), __float_as_int(rf.y), __float_as_int(rf.z), __float_as_int(rf.w)};
     float tn[4];
     bool hit[4];
@@ -310,12 +341,11 @@ MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, cons
     return step;
 }
 
-// LAY: MC_BVH_LAYOUT_BINARY, _WIDE4 or _WIDE4Q.
+// LAY: MC_BVH_LAYOUT_BINARY, _WIDE4, _WIDE4Q or MC_LAYOUT_OCTANT.
 template <bool ANY, int ISECT, bool COUNT, int LAY, class Stack>
 MC_D int trav_step_layout(const TraceScene& sc, TravState& s, const Stack& stack, const WatertightRay& w, int* err,
                           TravCount* cnt) {
-    if (LAY == MC_BVH_LAYOUT_WIDE4Q) return trav_step4<ANY, ISECT, COUNT, Stack, true>(sc, s, stack, w, err, cnt);
-    if (LAY == MC_BVH_LAYOUT_WIDE4) return trav_step4<ANY, ISECT, COUNT, Stack, false>(sc, s, stack, w, err, cnt);
+    if (LAY != MC_BVH_LAYOUT_BINARY) return trav_step4<ANY, ISECT, COUNT, Stack, LAY>(sc, s, stack, w, err, cnt);
     return trav_step<ANY, ISECT, COUNT, Stack>(sc, s, stack, w, err, cnt);
 }
 
