@@ -1,5 +1,5 @@
 """Builds at the sizes where the cooperative clustering and collapse change how
-they divide their work (tiles of 256, the rounds one block runs alone, blocks
+they divide their work (tiles of 240, the rounds one block runs alone, blocks
 with several scenes): the same tree, byte for byte, as the launch-per-phase
 loops, and the same scene bounds and hits as a build that also refits the LBVH."""
 import ctypes as C
