@@ -1936,7 +1936,8 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
     const bool smallWave = pathsOk && !guide && capacity <= fewPaths;
     // the first bounce k_paths may take over: guided bounces shade with the
     // guide, and a guided wave's second trace keeps the primary vertices'
-    // next-event estimates apart
+    // next-event estimates apart (a deep wave hands over at its read-backs, from
+    // the same bounce on)
     const int handFrom = !guide ? 1 : guidedDepth > 0 ? std::max(guidedDepth, 2) : maxD;
     const bool handOver = pathsOk && !deep && !smallWave && handFrom < maxD;
     auto enqueue_paths = [&](int lo, int hi, int few) {
@@ -2071,7 +2072,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
                 int next = 0;
                 MC_CUDA(cudaMemcpyAsync(&next, slot(d + 1), sizeof(int), cudaMemcpyDeviceToHost, stream));
                 MC_CUDA(cudaStreamSynchronize(stream));
-                few = pathsOk && next > 0 && next <= fewPaths;
+                few = pathsOk && d + 1 >= handFrom && next > 0 && next <= fewPaths;
                 stop = next == 0 || few;
             }
         }
