@@ -2,6 +2,7 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <string>
 #include <vector>
 
 #include "mc_abi.h"
@@ -123,7 +124,7 @@ struct mc_context {
     int scene_of_capacity = 0;
     cudaStream_t own_stream = nullptr;   // capture stream when the context has none
     void* graph_exec = nullptr;          // cached per-wave CUDA graph
-    unsigned long long graph_key[16] = {};  // every value the captured launches bake in
+    std::string graph_key;               // every value the captured launches bake in
     void* staging = nullptr;             // pinned host staging for large pageable uploads
     size_t staging_bytes = 0;
     // launch configurations measured on this context's device (occupancy of a

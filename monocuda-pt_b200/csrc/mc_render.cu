@@ -1597,7 +1597,7 @@ mc_status ensure_wave(mc_context* ctx, int capacity) {
     if (ctx->graph_exec) {
         cudaGraphExecDestroy((cudaGraphExec_t)ctx->graph_exec);
         ctx->graph_exec = nullptr;
-        std::memset(ctx->graph_key, 0, sizeof(ctx->graph_key));
+        ctx->graph_key.clear();
     }
     return MC_OK;
 }
@@ -1617,7 +1617,7 @@ static mc_status ensure_tables(mc_context* ctx, int capacity) {
         if (ctx->graph_exec) {
             cudaGraphExecDestroy((cudaGraphExec_t)ctx->graph_exec);
             ctx->graph_exec = nullptr;
-            std::memset(ctx->graph_key, 0, sizeof(ctx->graph_key));
+            ctx->graph_key.clear();
         }
     }
     return MC_OK;
@@ -1804,6 +1804,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
     unsigned short* sceneOf = n > 1 ? ctx->scene_of : nullptr;
 
     CameraArgs ca;
+    std::memset(&ca, 0, sizeof(ca));
     ca.tab = dtab;
     ca.sceneOf = sceneOf;
     ca.ox = w.ox; ca.oy = w.oy; ca.oz = w.oz; ca.dx = w.dx; ca.dy = w.dy; ca.dz = w.dz; ca.time = w.time;
@@ -2119,31 +2120,22 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
 
     cudaGraphExec_t exec = nullptr;
     if (useGraph) {
-        // the captured launches bake in these values; any change needs a new capture
-        unsigned long long key[16] = {(unsigned long long)(uintptr_t)stream,
-                                      (unsigned long long)capacity,
-                                      (unsigned long long)maxD,
-                                      (unsigned long long)((layout << 6) | (medium ? 2 : 0) | (philox ? 4 : 0) |
-                                                           (persistent ? 8 : 0) | (n > 1 ? 16 : 0) |
-                                                           (sameScene ? 32 : 0) | (grid ? 1024 : 0) | (smallWave ? 2048 : 0) | (handOver ? 4096 : 0)),
-                                      (unsigned long long)isect,
-                                      (unsigned long long)ta.refill,
-                                      (unsigned long long)(uintptr_t)ta.ts0.nodes,
-                                      (unsigned long long)(uintptr_t)ta.ts0.prims,
-                                      (unsigned long long)ta.ts0.root,
-                                      (unsigned long long)ta.medium0,
-                                      (unsigned long long)(uintptr_t)ta.cold0,
-                                      (unsigned long long)(uintptr_t)ta.spheres0,
-                                      (unsigned long long)(uintptr_t)w.block.ptr,
-                                      (unsigned long long)(uintptr_t)sceneOf,
-                                      (unsigned long long)(uintptr_t)dtab,
-                                      1ull};
-        if (ctx->graph_exec && std::memcmp(ctx->graph_key, key, sizeof(key)) == 0) {
+        // the captured launches bake in their whole argument structures (all
+        // cleared before they are filled, so their bytes compare) and these
+        // choices of kernel, grid and sequence; any change needs a new capture
+        const long long choices[] = {(long long)(uintptr_t)stream, capacity, maxD, w.capacity, layout, medium, grid, philox,
+                                     persistent, isect, n > 1, alias, smallWave, handOver, handFrom};
+        std::string key((const char*)choices, sizeof(choices));
+        key.append((const char*)&ca, sizeof(ca));
+        key.append((const char*)&sa, sizeof(sa));
+        key.append((const char*)&ta, sizeof(ta));
+        key.append((const char*)&ra, sizeof(ra));
+        if (ctx->graph_exec && ctx->graph_key == key) {
             exec = (cudaGraphExec_t)ctx->graph_exec;
         } else {
             if (ctx->graph_exec) cudaGraphExecDestroy((cudaGraphExec_t)ctx->graph_exec);
             ctx->graph_exec = nullptr;
-            std::memset(ctx->graph_key, 0, sizeof(ctx->graph_key));
+            ctx->graph_key.clear();
             cudaGraph_t graph;
             MC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
             mc_status cs = enqueue_wave();
@@ -2154,7 +2146,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
             cudaGraphDestroy(graph);
             if (ce != cudaSuccess) return cuda_error((int)ce, "cudaGraphInstantiate", __FILE__, __LINE__);
             ctx->graph_exec = exec;
-            std::memcpy(ctx->graph_key, key, sizeof(key));
+            ctx->graph_key = key;
         }
         launches = 0;
     }
