@@ -1280,7 +1280,14 @@ mc_status radix_sort_pairs_static(mc_context* ctx, uint32_t* keys, int32_t* vals
 }
 
 // Build buffers come from the device's stream-ordered pool (pool_alloc): they
-// are taken and returned in stream order, without a device-wide wait.
+// are taken and returned in stream order, without a device-wide wait. A build
+// takes one block for its work and one for what the tree keeps, then the wide
+// nodes, whose number it finds out, and returns the work block last. All of a
+// build's memory is then in use at once, and the next build finds the places of
+// this one's blocks free and whole. With some twenty buffers, taken and returned
+// at different times, the pool had more address ranges in rotation than memory
+// behind them and mapped memory from one to another inside warm builds: 5 to
+// 2,000 ms for a 4.8M-triangle batch that takes 3.6 ms.
 template <class T>
 static bool palloc(mc_context* ctx, T** p, size_t bytes) {
     void* v = nullptr;
@@ -1288,6 +1295,18 @@ static bool palloc(mc_context* ctx, T** p, size_t bytes) {
     *p = (T*)v;
     return ok;
 }
+
+// Hands out the parts of a block: first to add up their sizes (from null),
+// then from the allocation. 256-byte parts, as separate allocations have.
+struct Carver {
+    char* base = nullptr;
+    size_t used = 0;
+    template <class T>
+    void take(T*& p, size_t bytes) {
+        p = base ? (T*)(base + used) : nullptr;
+        used += (bytes + 255) & ~(size_t)255;
+    }
+};
 
 mc_status bvh_depth(mc_bvh* bvh) {
     if (bvh->depth >= 0) return MC_OK;
@@ -1796,7 +1815,7 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_rounds(PlocRounds a) {
 struct ClusterTree {
     float4* nodes = nullptr;
     std::vector<int> roots;
-    const int* deviceRoots = nullptr;  // in the nodes' allocation
+    const int* deviceRoots = nullptr;  // in the clustering's work
 };
 
 // The box of each scene's root: its two children's.
@@ -1807,41 +1826,42 @@ __global__ void k_root_boxes(const float4* __restrict__ nodes, const int* __rest
     boxes[s] = to_aabb(merge_box(load_child_box(nodes, roots[s], 0), load_child_box(nodes, roots[s], 1)));
 }
 
+// What the clustering works on.
+struct PlocWork {
+    int* cref[2];
+    float4* cbox[2];
+    int* nn;
+    int2 *flags, *pos, *sums;
+    int2* total;  // the round's totals, then [2..3] as ints: clusters, next node id
+    void carve(Carver& c, int N, int sms) {
+        const int per = kPlocBlock * kScanItems;
+        // tile sums of the per-phase launches, block sums of the cooperative one
+        const long long nbMax = std::max<long long>((N + per - 1) / per, 32ll * sms);
+        for (int*& p : cref) c.take(p, (size_t)N * 4);
+        for (float4*& p : cbox) c.take(p, (size_t)N * 32);
+        c.take(nn, (size_t)N * 4);
+        c.take(flags, (size_t)N * 8);
+        c.take(pos, (size_t)N * 8);
+        c.take(sums, (size_t)(nbMax + 1) * 8);
+        c.take(total, 32);
+    }
+};
+
 static mc_status build_ploc(mc_context* ctx, const mc_bvh* bvh, const Seg* dSeg, int nseg, const int32_t* order,
-                            const mc_aabb* bounds, ClusterTree& tree, bool coop) {
+                            const mc_aabb* bounds, const PlocWork& work, ClusterTree& tree, bool coop) {
     const int N = bvh->n, NI = bvh->ni;
     if (NI <= 0 || N < 2) return MC_ERR_UNSUPPORTED;
     const int per = kPlocBlock * kScanItems;
-    // tile sums of the per-phase launches, block sums of the cooperative one
-    const long long nbMax = std::max<long long>((N + per - 1) / per, 32ll * ctx->sm_count);
-    const size_t bytes = (size_t)NI * 64 + 2 * (size_t)N * 4 + 4 * (size_t)N * 16 + (size_t)N * 4 + 2 * (size_t)N * 8 +
-                         (size_t)(nbMax + 1) * 8 + 32 + 16 * 16;  // + the 16-byte rounding of each part
-    char* mem = nullptr;
-    if (!palloc(ctx, &mem, bytes)) {
-        cudaGetLastError();
-        return set_error(MC_ERR_OOM, "mc_bvh_build: clustering scratch allocation failed");
-    }
-    char* p = mem;
-    auto take = [&](size_t b) { char* r = p; p += (b + 15) & ~(size_t)15; return r; };
-    tree.nodes = (float4*)take((size_t)NI * 64);
-    int* cref[2] = {(int*)take((size_t)N * 4), (int*)take((size_t)N * 4)};
-    float4* cbox[2] = {(float4*)take((size_t)N * 32), (float4*)take((size_t)N * 32)};
-    int* nn = (int*)take((size_t)N * 4);
-    int2* flags = (int2*)take((size_t)N * 8);
-    int2* pos = (int2*)take((size_t)N * 8);
-    int2* sums = (int2*)take((size_t)(nbMax + 1) * 8);
-    int2* total = (int2*)take(32);  // the round's totals, then [2..3] as ints: clusters, next node id
-    auto fail = [&](mc_status s) {
-        pool_free(ctx, mem);
-        tree.nodes = nullptr;
-        return s;
-    };
+    int* const cref[2] = {work.cref[0], work.cref[1]};
+    float4* const cbox[2] = {work.cbox[0], work.cbox[1]};
+    int* nn = work.nn;
+    int2 *flags = work.flags, *pos = work.pos, *sums = work.sums, *total = work.total;
     const int loop = ctx->sm_count * 8;
     int* state = (int*)(total + 2);  // [0] clusters, [1] next node id
     k_ploc_init<<<std::min(grid_for(N, kBlock), loop), kBlock, 0, ctx->stream>>>(order, bounds, dSeg, nseg, N, cref[0], cbox[0]);
     const int h0[2] = {N, 0};
     if (cudaMemcpyAsync(state, h0, sizeof(h0), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
-        return fail(cuda_error(cudaGetLastError(), "mc_bvh_build (clustering)", __FILE__, __LINE__));
+        return cuda_error(cudaGetLastError(), "mc_bvh_build (clustering)", __FILE__, __LINE__);
     int n = N, nodeBase = 0, cur = 0, rounds = 0;
     // every round in one cooperative launch where the device supports it
     int coopAttr = 0, perSm = 0;
@@ -1861,10 +1881,10 @@ static mc_status build_ploc(mc_context* ctx, const mc_bvh* bvh, const Seg* dSeg,
             int h[4];
             if (cudaMemcpyAsync(h, state, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
                 cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-                return fail(cuda_error(cudaGetLastError(), "mc_bvh_build (clustering)", __FILE__, __LINE__));
+                return cuda_error(cudaGetLastError(), "mc_bvh_build (clustering)", __FILE__, __LINE__);
             int fl = 0;
             mc_status fs = flags_now(ctx, &fl);
-            if (fs != MC_OK || fl) return fail(fs != MC_OK ? fs : status_from_device_flags(fl));
+            if (fs != MC_OK || fl) return fs != MC_OK ? fs : status_from_device_flags(fl);
             n = h[0];
             nodeBase = h[1];
             cur = h[2];
@@ -1877,7 +1897,7 @@ static mc_status build_ploc(mc_context* ctx, const mc_bvh* bvh, const Seg* dSeg,
     // cluster count from the device and is sized for the last count seen
     const int kBatch = 8;
     while (n > nseg) {
-        if (rounds > 4096) return fail(set_error(MC_ERR_INVALID, "mc_bvh_build: clustering did not converge"));
+        if (rounds > 4096) return set_error(MC_ERR_INVALID, "mc_bvh_build: clustering did not converge");
         const int nb = (n + per - 1) / per;
         for (int r = 0; r < kBatch; r++, rounds++) {
             k_ploc_nn<<<(n + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, ctx->stream>>>(cbox[cur], state, nn);
@@ -1893,35 +1913,50 @@ static mc_status build_ploc(mc_context* ctx, const mc_bvh* bvh, const Seg* dSeg,
         int h[2];
         if (cudaMemcpyAsync(h, state, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
             cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-            return fail(cuda_error(cudaGetLastError(), "mc_bvh_build (clustering)", __FILE__, __LINE__));
+            return cuda_error(cudaGetLastError(), "mc_bvh_build (clustering)", __FILE__, __LINE__);
         int fl = 0;
         mc_status fs = flags_now(ctx, &fl);
-        if (fs != MC_OK || fl) return fail(fs != MC_OK ? fs : status_from_device_flags(fl));
+        if (fs != MC_OK || fl) return fs != MC_OK ? fs : status_from_device_flags(fl);
         n = h[0];
         nodeBase = h[1];
     }
     tree.roots.assign((size_t)nseg, -1);
     if (cudaMemcpyAsync(tree.roots.data(), cref[cur], (size_t)nseg * 4, cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-        return fail(cuda_error(cudaGetLastError(), "mc_bvh_build (clustering)", __FILE__, __LINE__));
+        return cuda_error(cudaGetLastError(), "mc_bvh_build (clustering)", __FILE__, __LINE__);
     int flagsNow = 0;
     mc_status st = flags_now(ctx, &flagsNow);
-    if (st != MC_OK || flagsNow) return fail(st != MC_OK ? st : status_from_device_flags(flagsNow));
-    if (nodeBase != NI || n != nseg) return fail(set_error(MC_ERR_INVALID, "mc_bvh_build: clustering left %d clusters", n));
+    if (st != MC_OK || flagsNow) return st != MC_OK ? st : status_from_device_flags(flagsNow);
+    if (nodeBase != NI || n != nseg) return set_error(MC_ERR_INVALID, "mc_bvh_build: clustering left %d clusters", n);
     for (int r : tree.roots)
-        if (r < 0) return fail(MC_ERR_UNSUPPORTED);  // a scene of one primitive: keep the LBVH
+        if (r < 0) return MC_ERR_UNSUPPORTED;  // a scene of one primitive: keep the LBVH
     tree.deviceRoots = cref[cur];
-    // the node block starts the allocation, so freeing it frees everything
     return MC_OK;
 }
+
+// What the collapse works on.
+struct WideWork {
+    int* rootOf;    // binary root of each wide node
+    int* front[2];
+    int* cnt;       // [0]: next frontier size; [4..8]: the cooperative collapse's results; [16..]: its block totals
+    int4* internal; // per frontier node: its internal slots
+    int* blockTotals;
+    void carve(Carver& c, int NI, int sms) {
+        c.take(rootOf, (size_t)NI * sizeof(int));
+        for (int*& p : front) c.take(p, (size_t)NI * sizeof(int));
+        c.take(cnt, (size_t)(16 + 32 * sms) * sizeof(int));
+        c.take(internal, (size_t)NI * sizeof(int4));
+        c.take(blockTotals, (size_t)(grid_for(NI, kBlock) + 1) * sizeof(int));
+    }
+};
 
 // The 4-wide collapse of a binary tree: `tree` (binary node layout, NI
 // internal nodes) with scene roots `roots`; the LBVH when tree is null. A
 // clustered tree whose greedy collapse would outgrow the traversal stack
 // returns MC_ERR_UNSUPPORTED (the caller then collapses the LBVH, which has
 // the depth-parity fallback).
-static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int nseg, int* dWideRoot, bool coop,
-                            const float4* tree = nullptr, const std::vector<int>* roots = nullptr) {
+static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int nseg, int* dWideRoot,
+                            const WideWork& work, bool coop, const float4* tree = nullptr, const std::vector<int>* roots = nullptr) {
     const int N = bvh->n, NI = bvh->ni;
     const float4* bin = tree ? tree : (const float4*)bvh->nodes;
     mc_status st;
@@ -1935,31 +1970,14 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
                                                                 (const int2*)ctx->scratch[1].ptr, dSeg, nseg, N, NI, rank,
                                                                 ctx->d_error);
     int count = 1;
-    int* rootOf = nullptr;   // greedy collapse: binary root of each wide node
+    int* rootOf = work.rootOf;
     bool greedy = false;
     if (NI > 0) {
         // surface-area-greedy collapse, level by level from the scene roots
-        int* front[2] = {nullptr, nullptr};
-        int* cnt = nullptr;  // [0]: next frontier size; [4..8]: the cooperative collapse's results; [16..]: its block totals
-        int4* internal = nullptr;  // per frontier node: its internal slots
-        int* blockTotals = nullptr;
-        auto release = [&]() {
-            pool_free(ctx, front[0]);
-            pool_free(ctx, front[1]);
-            pool_free(ctx, cnt);
-            pool_free(ctx, internal);
-            pool_free(ctx, blockTotals);
-        };
-        if (!palloc(ctx, &rootOf, (size_t)NI * sizeof(int)) ||
-            !palloc(ctx, &front[0], (size_t)NI * sizeof(int)) ||
-            !palloc(ctx, &front[1], (size_t)NI * sizeof(int)) || !palloc(ctx, &cnt, (size_t)(16 + 32 * ctx->sm_count) * sizeof(int)) ||
-            !palloc(ctx, &internal, (size_t)NI * sizeof(int4)) ||
-            !palloc(ctx, &blockTotals, (size_t)(grid_for(NI, kBlock) + 1) * sizeof(int))) {
-            cudaGetLastError();
-            release();
-            pool_free(ctx, rootOf);
-            return set_error(MC_ERR_OOM, "mc_bvh_build: wide-collapse scratch allocation failed");
-        }
+        int* const front[2] = {work.front[0], work.front[1]};
+        int* cnt = work.cnt;
+        int4* internal = work.internal;
+        int* blockTotals = work.blockTotals;
         MC_CUDA(cudaMemsetAsync(wideId, 0xFF, (size_t)NI * sizeof(int), ctx->stream));
         const std::vector<int> rootList = roots ? *roots : std::vector<int>(bvh->bin_roots.begin(), bvh->bin_roots.end());
         MC_CUDA(cudaMemcpyAsync(front[0], rootList.data(), rootList.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
@@ -1991,11 +2009,8 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
                 int h[4];
                 MC_CUDA(cudaMemcpyAsync(h, cnt + 4, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
                 MC_CUDA(cudaStreamSynchronize(ctx->stream));
-                if (h[3]) {
-                    release();
-                    pool_free(ctx, rootOf);
+                if (h[3])
                     return set_error(MC_ERR_INVALID, "mc_bvh_build: the collapse found more nodes than internal nodes");
-                }
                 levels = h[0];
                 idBase = h[1];
                 n = h[2];
@@ -2012,34 +2027,20 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
                                                                    wideId, ctx->d_error);
             MC_CUDA(cudaMemcpyAsync(&n, cnt, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
             MC_CUDA(cudaStreamSynchronize(ctx->stream));
-            if (n < 0 || (long long)idBase + n > NI) {
-                // more wide nodes than internal nodes: not a binary tree over these leaves
-                release();
-                pool_free(ctx, rootOf);
+            if (n < 0 || (long long)idBase + n > NI)  // more wide nodes than internal nodes: not a binary tree over these leaves
                 return set_error(MC_ERR_INVALID, "mc_bvh_build: the collapse found %d nodes past %d", n, idBase);
-            }
             idBase += n;
             cur = 1 - cur;
             levels++;
         }
         count = idBase;
         int flags = 0;
-        if ((st = flags_now(ctx, &flags)) != MC_OK || flags) {
-            release();
-            pool_free(ctx, rootOf);
-            return st != MC_OK ? st : status_from_device_flags(flags);
-        }
-        release();
+        if ((st = flags_now(ctx, &flags)) != MC_OK || flags) return st != MC_OK ? st : status_from_device_flags(flags);
         // a visit pushes at most 3 siblings: the traversal stack must hold 3 per level
         greedy = n == 0 && 3 * levels <= MC_STACK_CAPACITY;
         bvh->wide_levels = greedy ? levels : -1;
-        if (!greedy && tree) {
-            pool_free(ctx, rootOf);
-            return MC_ERR_UNSUPPORTED;
-        }
+        if (!greedy && tree) return MC_ERR_UNSUPPORTED;
         if (!greedy) {
-            pool_free(ctx, rootOf);
-            rootOf = nullptr;
             MC_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), ctx->stream));
             k_wide_select<<<grid_for(NI, kBlock), kBlock, 0, ctx->stream>>>(bvh->parents, dSeg, nseg, NI, wideId, counter,
                                                                            dWideRoot);
@@ -2047,14 +2048,9 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
         }
     }
     int flags = 0;
-    if ((st = flags_now(ctx, &flags)) != MC_OK || flags) {
-        pool_free(ctx, rootOf);
-        return st != MC_OK ? st : status_from_device_flags(flags);
-    }
-    if (!palloc(ctx, &bvh->wide_nodes, (size_t)count * 128) ||
-        !palloc(ctx, &bvh->records, (size_t)N * 64)) {
+    if ((st = flags_now(ctx, &flags)) != MC_OK || flags) return st != MC_OK ? st : status_from_device_flags(flags);
+    if (!palloc(ctx, &bvh->wide_nodes, (size_t)count * 128)) {
         cudaGetLastError();
-        pool_free(ctx, rootOf);
         return set_error(MC_ERR_OOM, "mc_bvh_build: wide-node allocation failed");
     }
     bvh->wide_roots.assign(nseg, 0);
@@ -2062,8 +2058,6 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
         k_wide_fill_greedy<<<grid_for(count, kBlock), kBlock, 0, ctx->stream>>>(bin, rootOf, wideId,
                                                                               rank, count, (float4*)bvh->wide_nodes);
         for (int s = 0; s < nseg; s++) bvh->wide_roots[s] = s;
-        MC_CUDA(cudaStreamSynchronize(ctx->stream));
-        pool_free(ctx, rootOf);
     } else if (NI > 0) {
         k_wide_fill<<<grid_for(NI, kBlock), kBlock, 0, ctx->stream>>>((const float4*)bvh->nodes, wideId, rank, NI,
                                                                      (float4*)bvh->wide_nodes);
@@ -2124,21 +2118,54 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
     auto fail = [&](mc_status s) { mc_bvh_free(bvh); return s; };
 
     long long nodesCount = std::max(1, NI);
-    if (!palloc(ctx, &bvh->nodes, (size_t)nodesCount * 64) ||
-        !palloc(ctx, &bvh->prims, (size_t)N * 48) ||
-        !palloc(ctx, &bvh->codes, (size_t)N * 4) ||
-        !palloc(ctx, &bvh->ids, (size_t)N * 4) ||
-        !palloc(ctx, &bvh->types, (size_t)N * 4) ||
-        !palloc(ctx, &bvh->parents, (size_t)(NI + N) * 4 + 8)) {
+    const bool wide = o.layout == MC_BVH_LAYOUT_WIDE4 || o.layout == MC_BVH_LAYOUT_WIDE4Q;
+    const bool clustered = wide && o.builder == MC_BVH_BUILDER_CLUSTERED;
+    // the build's work: the primitives in leaf order and, for the wide layouts,
+    // the LBVH's nodes and the clustered ones; then one place for the batch
+    // sort's arrays, the clustering and the collapse in turn (the collapse no
+    // longer reads what the clustering left there)
+    uint32_t* sortKeys;
+    int32_t* sortValues;
+    float4* clusterNodes;
+    PlocWork ploc;
+    WideWork collapse;
+    auto carve_work = [&](Carver c) {
+        c.take(bvh->prims, (size_t)N * 48);
+        if (wide) c.take(bvh->nodes, (size_t)nodesCount * 64);
+        if (clustered) c.take(clusterNodes, (size_t)nodesCount * 64);
+        Carver sort = c, cluster = c, fold = c;
+        if (nseg > 1) {
+            sort.take(sortKeys, (size_t)N * 4);
+            sort.take(sortValues, (size_t)N * 4);
+        }
+        if (clustered) ploc.carve(cluster, N, ctx->sm_count);
+        if (wide) collapse.carve(fold, NI, ctx->sm_count);
+        return std::max({sort.used, cluster.used, fold.used});
+    };
+    auto carve_block = [&](Carver c) {
+        c.take(bvh->records, (size_t)N * 64);
+        if (!wide) c.take(bvh->nodes, (size_t)nodesCount * 64);
+        c.take(bvh->codes, (size_t)N * 4);
+        c.take(bvh->ids, (size_t)N * 4);
+        c.take(bvh->types, (size_t)N * 4);
+        c.take(bvh->parents, (size_t)(NI + N) * 4 + 8);
+        return c.used;
+    };
+    const size_t workBytes = carve_work(Carver()), blockBytes = carve_block(Carver());
+    if (!palloc(ctx, &bvh->work, workBytes) || !palloc(ctx, &bvh->block, blockBytes)) {
         cudaGetLastError();
         return fail(set_error(MC_ERR_OOM, "mc_bvh_build: device allocation failed (n=%d)", N));
     }
+    carve_work(Carver{(char*)bvh->work});
+    carve_block(Carver{(char*)bvh->block});
+    bvh->device_bytes = (long long)blockBytes;
     if (o.keep_reference_nodes) {
         if (!palloc(ctx, &bvh->ref_internal, (size_t)nodesCount * sizeof(mc_bvh_node)) ||
             !palloc(ctx, &bvh->ref_leaves, (size_t)N * sizeof(mc_bvh_node))) {
             cudaGetLastError();
             return fail(set_error(MC_ERR_OOM, "mc_bvh_build: device allocation failed (reference nodes)"));
         }
+        bvh->device_bytes += (nodesCount + (long long)N) * (long long)sizeof(mc_bvh_node);
         cudaMemsetAsync(bvh->ref_internal, 0, (size_t)nodesCount * sizeof(mc_bvh_node), ctx->stream);
         cudaMemsetAsync(bvh->ref_leaves, 0, (size_t)N * sizeof(mc_bvh_node), ctx->stream);
     }
@@ -2193,17 +2220,7 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
             k_segment_keys<<<grid_for(N, kBlock), kBlock, 0, ctx->stream>>>(centroids, order, N, segKeys);
             int bits = 1;
             while ((1 << bits) < nseg) bits++;
-            // the sort needs its own two scratch arrays: reuse the node buffer (>= N-1 ints) is not enough, so allocate
-            uint32_t* altK = nullptr;
-            int32_t* altV = nullptr;
-            if (!palloc(ctx, &altK, (size_t)N * 4) || !palloc(ctx, &altV, (size_t)N * 4)) {
-                cudaGetLastError();
-                pool_free(ctx, altK);
-                return fail(set_error(MC_ERR_OOM, "mc_bvh_build_batch: sort scratch allocation failed"));
-            }
-            st = radix_sort_pairs(ctx, segKeys, order, altK, altV, N, bits);
-            pool_free(ctx, altK);
-            pool_free(ctx, altV);
+            st = radix_sort_pairs(ctx, segKeys, order, sortKeys, sortValues, N, bits);
             if (st != MC_OK) return fail(st);
             k_gather_u32<<<grid_for(N, kBlock), kBlock, 0, ctx->stream>>>(codesRef, order, N, bvh->codes, ctx->d_error);
         }
@@ -2227,8 +2244,7 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
     // and a collapse of the LBVH read; a clustered tree needs its topology alone
     // (leaf ranks), and its own root box is the scene's: at 1M triangles the
     // refit is 200 us of a build.
-    const bool wide = o.layout == MC_BVH_LAYOUT_WIDE4 || o.layout == MC_BVH_LAYOUT_WIDE4Q;
-    const bool clusteredOnly = wide && o.builder == MC_BVH_BUILDER_CLUSTERED && !o.keep_reference_nodes && N > 1;
+    const bool clusteredOnly = clustered && !o.keep_reference_nodes && N > 1;
     bvh->seg_bounds.resize(nseg);
     auto leaves = [&](bool boxes) -> mc_status {
         k_leaves_refit<<<grid_for(N, kBlock), kBlock, 0, ctx->stream>>>(order, boundsRef, N, NI, dSeg, nseg, (float4*)bvh->nodes,
@@ -2261,27 +2277,21 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
         // the LBVH when clustering does not apply (a one-primitive scene, a
         // collapse too deep for the stack) or the caller asks for it
         st = MC_ERR_UNSUPPORTED;
-        if (o.builder == MC_BVH_BUILDER_CLUSTERED) {
+        if (clustered) {
             ClusterTree tree;
-            st = build_ploc(ctx, bvh, dSeg, nseg, order, boundsRef, tree, coop);
+            tree.nodes = clusterNodes;
+            st = build_ploc(ctx, bvh, dSeg, nseg, order, boundsRef, ploc, tree, coop);
             if (st == MC_OK && clusteredOnly) {
                 k_root_boxes<<<grid_for(nseg, kBlock), kBlock, 0, ctx->stream>>>(tree.nodes, tree.deviceRoots, nseg, dRootBoxes);
-                if ((st = root_boxes()) != MC_OK) {
-                    pool_free(ctx, tree.nodes);
-                    return fail(st);
-                }
+                if ((st = root_boxes()) != MC_OK) return fail(st);
             }
             if (st == MC_OK) {
-                st = build_wide(ctx, bvh, dSeg, nseg, dWideRoot, coop, tree.nodes, &tree.roots);
-                pool_free(ctx, tree.nodes);
+                st = build_wide(ctx, bvh, dSeg, nseg, dWideRoot, collapse, coop, tree.nodes, &tree.roots);
                 if (st == MC_OK) bvh->builder = MC_BVH_BUILDER_CLUSTERED;
             }
             if (st != MC_OK && st != MC_ERR_UNSUPPORTED) return fail(st);
         }
         if (st == MC_ERR_UNSUPPORTED) {
-            if (bvh->wide_nodes) pool_free(ctx, bvh->wide_nodes);
-            if (bvh->records) pool_free(ctx, bvh->records);
-            bvh->wide_nodes = bvh->records = nullptr;
             if (clusteredOnly) {
                 if ((st = devbuf_reserve(ctx->scratch[5], (size_t)nodesCount * 4 + 16)) != MC_OK) return fail(st);
                 counters = (int*)ctx->scratch[5].ptr;
@@ -2289,7 +2299,7 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
                     return fail(cuda_error(cudaGetLastError(), "memset", __FILE__, __LINE__));
                 if ((st = leaves(true)) != MC_OK || (st = root_boxes()) != MC_OK) return fail(st);
             }
-            if ((st = build_wide(ctx, bvh, dSeg, nseg, dWideRoot, coop)) != MC_OK) return fail(st);
+            if ((st = build_wide(ctx, bvh, dSeg, nseg, dWideRoot, collapse, coop)) != MC_OK) return fail(st);
             bvh->builder = MC_BVH_BUILDER_LBVH;
         }
     }
@@ -2322,16 +2332,17 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
         }
     }
     if (bvh->layout == MC_BVH_LAYOUT_BINARY) {
-        if (!palloc(ctx, &bvh->records, (size_t)N * 64)) {
-            cudaGetLastError();
-            return fail(set_error(MC_ERR_OOM, "mc_bvh_build: leaf-record allocation failed"));
-        }
         if ((st = leaf_records(ctx, bvh->prims, nullptr, N, bvh->records)) != MC_OK) return fail(st);
         if (cudaStreamSynchronize(ctx->stream) != cudaSuccess)
             return fail(cuda_error(cudaGetLastError(), "mc_bvh_build (leaf records)", __FILE__, __LINE__));
     }
-    pool_free(ctx, bvh->prims);  // the records replace the build's primitive stream
-    bvh->prims = nullptr;
+    if (wide) {
+        bvh->device_bytes += bvh->wide_count * (bvh->layout == MC_BVH_LAYOUT_WIDE4Q ? 64 : 128) +
+                             (bvh->octant_nodes ? bvh->wide_count * 192 : 0);
+        bvh->nodes = nullptr;  // the build's: traversal reads the wide nodes
+    }
+    pool_free(ctx, bvh->work);
+    bvh->work = bvh->prims = nullptr;
     *out = bvh;
     return MC_OK;
 }
@@ -2415,8 +2426,7 @@ mc_status mc_bvh_free(mc_bvh* bvh) {
     if (prev != bvh->device) cudaSetDevice(bvh->device);
     // work on any stream may still read the tree (cudaFree would wait for the device too)
     cudaDeviceSynchronize();
-    void* bufs[] = {bvh->nodes, bvh->prims, bvh->wide_nodes, bvh->octant_nodes, bvh->records, bvh->codes,
-                    bvh->ids, bvh->types, bvh->parents, bvh->ref_internal, bvh->ref_leaves};
+    void* bufs[] = {bvh->wide_nodes, bvh->octant_nodes, bvh->block, bvh->work, bvh->ref_internal, bvh->ref_leaves};
     for (void* b : bufs) mc::pool_release(b);
     if (prev >= 0 && prev != bvh->device) cudaSetDevice(prev);
     delete bvh;

@@ -66,21 +66,28 @@ void devbuf_free(DevBuf& b) {
     b.bytes = 0;
 }
 
-// One stream-ordered memory pool per device for the BVH build's buffers. It
-// keeps what is freed (release threshold: never), so a build after the first
-// takes its memory without a driver allocation; plain cudaMalloc / cudaFree
-// pairs per build cost from well under a millisecond to hundreds of
-// milliseconds each. The pools live as long as the process: a tree may
-// outlive the context that built it.
+// Stream-ordered memory pools, two per device. The one for trees (and a
+// server's images) keeps what is freed (release threshold: never), so a build
+// after the first takes its memory without a driver allocation; plain
+// cudaMalloc / cudaFree pairs per build cost from well under a millisecond to
+// hundreds of milliseconds each. The other one, for the buffers of single
+// calls, keeps what one host render can take from it. They are apart because a
+// call's buffers would lie in the places a build looks for: the pool then maps
+// memory from one address range to another (5 to 36 ms of a 2.6 ms build after
+// two host renders). The pools live as long as the process: a tree may outlive
+// the context that built it.
 namespace {
 std::mutex g_pool_mutex;
-std::unordered_map<int, cudaMemPool_t> g_pools;
+enum { POOL_TREES = 0, POOL_CALLS = 1 };
+std::unordered_map<int, cudaMemPool_t> g_pools[2];
+constexpr size_t kCallPooled = (size_t)64 << 20;            // largest buffer of a call that is pooled
+constexpr unsigned long long kCallKept = 6 * kCallPooled;  // a host render has five buffers, its ingestion one
 }
 
-static cudaMemPool_t device_pool(int device) {
+static cudaMemPool_t device_pool(int device, int which) {
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    auto it = g_pools.find(device);
-    if (it != g_pools.end()) return it->second;
+    auto it = g_pools[which].find(device);
+    if (it != g_pools[which].end()) return it->second;
     cudaMemPoolProps props;
     std::memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
@@ -92,15 +99,15 @@ static cudaMemPool_t device_pool(int device) {
         cudaGetLastError();
         return nullptr;
     }
-    unsigned long long keep = ~0ull;
+    unsigned long long keep = which == POOL_CALLS ? kCallKept : ~0ull;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    g_pools[device] = pool;
+    g_pools[which][device] = pool;
     return pool;
 }
 
-mc_status pool_alloc(mc_context* ctx, void** p, size_t bytes) {
+static mc_status alloc_from(mc_context* ctx, int which, void** p, size_t bytes) {
     *p = nullptr;
-    cudaMemPool_t pool = device_pool(ctx->device);
+    cudaMemPool_t pool = device_pool(ctx->device, which);
     if (!pool) return set_error(MC_ERR_CUDA, "device %d: memory pool creation failed", ctx->device);
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes < 256 ? 256 : bytes, pool, ctx->stream);
     if (e != cudaSuccess) {
@@ -110,6 +117,8 @@ mc_status pool_alloc(mc_context* ctx, void** p, size_t bytes) {
     }
     return MC_OK;
 }
+
+mc_status pool_alloc(mc_context* ctx, void** p, size_t bytes) { return alloc_from(ctx, POOL_TREES, p, bytes); }
 
 void pool_free(mc_context* ctx, void* p) {
     if (p) cudaFreeAsync(p, ctx->stream);
@@ -121,14 +130,12 @@ void pool_release(void* p) {
     if (p) cudaFreeAsync(p, 0);
 }
 
-// A call's own device buffers, freed before it returns: from the pool up to
-// 64 MB each (a cudaMalloc and its cudaFree cost 0.3 to 1 ms and wait for the
-// device; the pool keeps no more than that for the next call), from cudaMalloc
-// above.
-constexpr size_t kCallPooled = (size_t)64 << 20;
-
+// A call's own device buffers, freed before it returns: pooled up to 64 MB
+// each (a cudaMalloc and its cudaFree cost 0.3 to 1 ms and wait for the device;
+// the pool keeps at most 384 MB between calls, until a context closes), from
+// cudaMalloc above.
 mc_status call_alloc(mc_context* ctx, void** p, size_t bytes) {
-    if (bytes <= kCallPooled) return pool_alloc(ctx, p, bytes);
+    if (bytes <= kCallPooled) return alloc_from(ctx, POOL_CALLS, p, bytes);
     *p = nullptr;
     if (cudaMalloc(p, bytes) != cudaSuccess) {
         cudaGetLastError();
@@ -145,8 +152,10 @@ void call_free(mc_context* ctx, void* p, size_t bytes) {
 
 void pool_trim(int device) {
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    auto it = g_pools.find(device);
-    if (it != g_pools.end()) cudaMemPoolTrimTo(it->second, 0);
+    for (auto& pools : g_pools) {
+        auto it = pools.find(device);
+        if (it != pools.end()) cudaMemPoolTrimTo(it->second, 0);
+    }
 }
 
 // One lane polls *flag (system-scope acquire loads, so a flag in mapped host

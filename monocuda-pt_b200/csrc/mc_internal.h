@@ -152,7 +152,12 @@ struct mc_bvh {
     int layout = MC_BVH_LAYOUT_BINARY;
     int builder = MC_BVH_BUILDER_LBVH;  // the binary tree the wide layout collapses
     int depth = -1;
-    void* nodes = nullptr;             // traversal nodes (float4 records)
+    // one allocation each: what the tree keeps (the arrays below point into it,
+    // but for the wide nodes and the reference nodes) and what only its build needs
+    void* block = nullptr;
+    void* work = nullptr;
+    long long device_bytes = 0;        // of all the tree's allocations
+    void* nodes = nullptr;             // binary nodes (float4 records); wide layouts: during the build
     long long node_count = 0;
     long long node_bytes = 0;
     void* prims = nullptr;             // during the build: leaf-ordered primitives, 48 B each
