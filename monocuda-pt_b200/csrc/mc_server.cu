@@ -48,16 +48,6 @@ struct ServerRequest {
     double submit_s = 0, admit_s = 0, done_s = 0;
 };
 
-// What a scene's BVH is charged against the budget: nodes, 96 bytes of leaf data
-// a primitive, codes and order. (The leaf records take 64 of the 96; the octant
-// nodes of a small tree, at most 50 MB, come out of the rest or beside it.)
-long long bvh_bytes(const mc_bvh* b) {
-    long long n = b->n;
-    long long s = b->node_bytes + n * 48 + b->wide_count * 128 + n * 48 + 3 * n * 4 + (2 * n) * 4;
-    if (b->ref_internal) s += (2 * n) * (long long)sizeof(mc_bvh_node);
-    return s;
-}
-
 }  // namespace
 
 struct mc_server {
@@ -157,7 +147,7 @@ mc_status mc_server_add_scene(mc_server* s, const mc_scene_view* scene, int64_t*
     sc.view = *scene;
     mc_status st = mc_bvh_build(s->ctx, scene, &opts, &sc.bvh);
     if (st != MC_OK) return st;
-    sc.bytes = bvh_bytes(sc.bvh);
+    sc.bytes = sc.bvh->device_bytes;
     if (s->used + sc.bytes > s->cfg.hbm_budget_bytes) {
         mc_bvh_free(sc.bvh);
         return mc::set_error(MC_ERR_BUDGET, "mc_server_add_scene: the scene's BVH (%lld bytes) does not fit the budget",
