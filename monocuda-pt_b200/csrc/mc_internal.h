@@ -27,6 +27,9 @@ typedef struct CUstream_st* cudaStream_t;
 // Traversal form of a launch whose trees all have octant nodes (the public
 // layouts are 0..2).
 #define MC_LAYOUT_OCTANT 3
+// Added to the form of a launch of 4-wide trees whose rays may need more stack
+// than there is: children are pushed in full order (trav_step4).
+#define MC_LAYOUT_ORDERED 4
 
 namespace mc {
 
@@ -130,10 +133,10 @@ struct mc_context {
     // launch configurations measured on this context's device (occupancy of a
     // kernel variant, its opt-in shared-memory size), filled on first use; a
     // context is used by one host thread at a time, so these need no lock
-    int trace_blocks[192] = {};
-    int trace_blocks_smem[192] = {};     // shared-memory bytes trace_blocks[k] was measured with
-    int trace_smem_attr[192] = {};       // dynamic shared memory the variant has been opted in to
-    int paths_blocks[4] = {};            // k_paths, per traversal form
+    int trace_blocks[384] = {};
+    int trace_blocks_smem[384] = {};     // shared-memory bytes trace_blocks[k] was measured with
+    int trace_smem_attr[384] = {};       // dynamic shared memory the variant has been opted in to
+    int paths_blocks[8] = {};            // k_paths, per traversal form
     int paths_blocks_smem = 0;           // shared-memory bytes they were measured with
     int shade_blocks[3] = {};            // Philox, XORWOW, guided
     bool guide_attrs_set = false;        // the guide kernels' shared-memory opt-in is done

@@ -1493,28 +1493,29 @@ int occupancy_blocks(const void* fn, int sms, size_t smem = 0, int threads = 256
 
 typedef void (*TraceKernel)(TraceArgs);
 
-// [batch][layout][count][medium kind][isect]
+// [batch][traversal form][count][medium kind][isect]; only 4-wide trees have ordered forms
 #define MC_TKM(C, L, B)                                                                                   \
     {{k_trace<0, 0, C, L, B>, k_trace<1, 0, C, L, B>}, {k_trace<0, 1, C, L, B>, k_trace<1, 1, C, L, B>}, \
      {k_trace<0, 2, C, L, B>, k_trace<1, 2, C, L, B>}}
 #define MC_TK(L, B) {MC_TKM(false, L, B), MC_TKM(true, L, B)}
 // medium: 0 none, 1 homogeneous media only, 2 media with density grids
-TraceKernel trace_kernel(bool batch, int layout, bool count, int medium, int isect) {
-    static const TraceKernel table[2][4][2][3][2] = {
-        {MC_TK(0, false), MC_TK(1, false), MC_TK(2, false), MC_TK(3, false)},
-        {MC_TK(0, true), MC_TK(1, true), MC_TK(2, true), MC_TK(3, true)}};
-    return table[batch ? 1 : 0][layout][count ? 1 : 0][medium][isect ? 1 : 0];
+TraceKernel trace_kernel(bool batch, int form, bool count, int medium, int isect) {
+    static const TraceKernel table[2][8][2][3][2] = {
+        {MC_TK(0, false), MC_TK(1, false), MC_TK(2, false), MC_TK(3, false), MC_TK(0, false), MC_TK(5, false),
+         MC_TK(6, false), MC_TK(7, false)},
+        {MC_TK(0, true), MC_TK(1, true), MC_TK(2, true), MC_TK(3, true), MC_TK(0, true), MC_TK(5, true), MC_TK(6, true),
+         MC_TK(7, true)}};
+    return table[batch ? 1 : 0][form][count ? 1 : 0][medium][isect ? 1 : 0];
 }
 // The 128-thread variant, compiled for launches of the reference intersector
-// without counters or density grids; [batch][layout][medium kind].
-#define MC_TK128(B)                                                                                     \
-    {{k_trace<0, 0, false, 0, B, 128>, k_trace<0, 1, false, 0, B, 128>},                                \
-     {k_trace<0, 0, false, 1, B, 128>, k_trace<0, 1, false, 1, B, 128>},                                \
-     {k_trace<0, 0, false, 2, B, 128>, k_trace<0, 1, false, 2, B, 128>},                                \
-     {k_trace<0, 0, false, 3, B, 128>, k_trace<0, 1, false, 3, B, 128>}}
-TraceKernel trace_kernel_128(bool batch, int layout, int medium) {
-    static const TraceKernel table[2][4][2] = {MC_TK128(false), MC_TK128(true)};
-    return table[batch ? 1 : 0][layout][medium];
+// without counters or density grids; [batch][traversal form][medium kind].
+#define MC_TK128L(L, B) {k_trace<0, 0, false, L, B, 128>, k_trace<0, 1, false, L, B, 128>}
+#define MC_TK128(B)                                                                                        \
+    {MC_TK128L(0, B), MC_TK128L(1, B), MC_TK128L(2, B), MC_TK128L(3, B), MC_TK128L(0, B), MC_TK128L(5, B), \
+     MC_TK128L(6, B), MC_TK128L(7, B)}
+TraceKernel trace_kernel_128(bool batch, int form, int medium) {
+    static const TraceKernel table[2][8][2] = {MC_TK128(false), MC_TK128(true)};
+    return table[batch ? 1 : 0][form][medium];
 }
 
 // Persistent: one wave of resident blocks (SMs x resident blocks per SM) that
@@ -1522,7 +1523,7 @@ TraceKernel trace_kernel_128(bool batch, int layout, int medium) {
 // one ray per thread and no refill, over plainBlocks blocks; sharing the kernel
 // keeps the per-ray arithmetic identical between the two modes. A launch is a
 // batch launch when it carries a per-path scene map.
-void launch_trace(mc_context* ctx, cudaStream_t stream, const TraceArgs& t0, int layout, int medium, int isect,
+void launch_trace(mc_context* ctx, cudaStream_t stream, const TraceArgs& t0, int form, int medium, int isect,
                   bool persistent, int plainBlocks, bool count = false) {
     TraceArgs t = t0;
     t.oneShot = persistent ? 0 : 1;
@@ -1533,9 +1534,9 @@ void launch_trace(mc_context* ctx, cudaStream_t stream, const TraceArgs& t0, int
     const int threads = small ? 128 : kTraceThreads;
     // the shared-memory stack holds stackCap entries per lane
     const int smem = threads * t.stackCap * (int)sizeof(int);
-    TraceKernel fn = small ? trace_kernel_128(batch, layout, medium) : trace_kernel(batch, layout, count, medium, isect);
-    const int key = medium + 3 * (isect ? 1 : 0) + 6 * (count ? 1 : 0) + 12 * (batch ? 1 : 0) + 24 * layout +
-                    96 * (small ? 1 : 0);  // < 192
+    TraceKernel fn = small ? trace_kernel_128(batch, form, medium) : trace_kernel(batch, form, count, medium, isect);
+    const int key = medium + 3 * (isect ? 1 : 0) + 6 * (count ? 1 : 0) + 12 * (batch ? 1 : 0) + 24 * form +
+                    192 * (small ? 1 : 0);  // < 384
     if (smem > 48 * 1024 && ctx->trace_smem_attr[key] < smem) {
         cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         ctx->trace_smem_attr[key] = smem;
@@ -1717,13 +1718,14 @@ constexpr int kPathsInFlightGrid = 1 << 20;
 // paths 939 -> 739 us, Cornell boxes 493 -> 423 us, 16 small scenes 2.16 -> 2.12 ms.
 constexpr int kHandOver = 1 << 14;
 
-static void launch_paths(mc_context* ctx, cudaStream_t stream, const ShadeArgs& a, PathsArgs v, int layout) {
+static void launch_paths(mc_context* ctx, cudaStream_t stream, const ShadeArgs& a, PathsArgs v, int form) {
     typedef void (*Kernel)(ShadeArgs, PathsArgs);
-    static const Kernel table[4] = {k_paths<0>, k_paths<1>, k_paths<2>, k_paths<3>};
-    const Kernel fn = table[layout];
+    static const Kernel table[8] = {k_paths<0>, k_paths<1>, k_paths<2>, k_paths<3>,
+                                    k_paths<0>, k_paths<5>, k_paths<6>, k_paths<7>};
+    const Kernel fn = table[form];
     if (v.stackCap <= 0 || v.stackCap > MC_STACK_CAPACITY) v.stackCap = MC_STACK_CAPACITY;
     const int smem = kPathsThreads * v.stackCap * (int)sizeof(int);  // at most 32 KB: no opt-in
-    int& blocks = ctx->paths_blocks[layout];
+    int& blocks = ctx->paths_blocks[form];
     if (!blocks || ctx->paths_blocks_smem != smem) {
         if (ctx->paths_blocks_smem != smem)
             for (int& b : ctx->paths_blocks) b = 0;
@@ -1842,14 +1844,15 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
     ta.queueCap = queueCap;
     ta.stackCap = p0.stack_entries;
     ta.threads = p0.trace_threads;
-    if (ta.threads == 0 && ta.stackCap == 0) {
-        int levels = 0;
-        for (int i = 0; i < n && levels >= 0; i++) {
-            const int l = shape_levels(items[i].bvh ? items[i].bvh : bvh);
-            levels = l < 0 ? -1 : std::max(levels, l);
-        }
-        default_shape(ta, levels, isect);
+    int levels = 0;
+    for (int i = 0; i < n && levels >= 0; i++) {
+        const int l = shape_levels(items[i].bvh ? items[i].bvh : bvh);
+        levels = l < 0 ? -1 : std::max(levels, l);
     }
+    if (ta.threads == 0 && ta.stackCap == 0) default_shape(ta, levels, isect);
+    // 3 entries per level, or MC_STACK_CAPACITY of them, hold what any ray pushes
+    const bool ordered = ta.stackCap > 0 && ta.stackCap < (levels > 0 ? 3 * levels : MC_STACK_CAPACITY);
+    const int form = layout | (ordered ? MC_LAYOUT_ORDERED : 0);
     ta.refill = (p0.refill_threshold > 0 && p0.refill_threshold <= 32) ? p0.refill_threshold : 8;  // PT:3400
     if (countVisits) ta.counts = (unsigned long long*)(ctx->d_stats + 2 * MC_MAX_DEPTH_STATS);
     if (sameScene) {
@@ -1955,7 +1958,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
         v.gridMedia = grid ? 1 : 0;
         v.stats = ctx->d_stats;
         v.err = ctx->d_error;
-        launch_paths(ctx, stream, sa, v, layout);
+        launch_paths(ctx, stream, sa, v, form);
         launches++;
     };
     auto enqueue_wave = [&]() -> mc_status {
@@ -1998,7 +2001,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
             }
             if (grid && d > 0) MC_CUDA(cudaMemsetAsync(ta.vdefer, 0, sizeof(int), stream));
             phaseBegin(0);
-            launch_trace(ctx, stream, t, layout, grid ? 2 : medium ? 1 : 0, isect, persistent, plainBlocks, countVisits);
+            launch_trace(ctx, stream, t, form, grid ? 2 : medium ? 1 : 0, isect, persistent, plainBlocks, countVisits);
             phaseEnd();
             launches++;
             if (grid && d > 0) {
@@ -2123,7 +2126,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
         // the captured launches bake in their whole argument structures (all
         // cleared before they are filled, so their bytes compare) and these
         // choices of kernel, grid and sequence; any change needs a new capture
-        const long long choices[] = {(long long)(uintptr_t)stream, capacity, maxD, w.capacity, layout, medium, grid, philox,
+        const long long choices[] = {(long long)(uintptr_t)stream, capacity, maxD, w.capacity, form, medium, grid, philox,
                                      persistent, isect, n > 1, alias, smallWave, handOver, handFrom};
         std::string key((const char*)choices, sizeof(choices));
         key.append((const char*)&ca, sizeof(ca));

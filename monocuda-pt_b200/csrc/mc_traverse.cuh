@@ -17,7 +17,7 @@
 
 namespace mc {
 
-enum { STEP_CONTINUE = 0, STEP_DONE = 1, STEP_OCCLUDED = 2 };
+enum { STEP_CONTINUE = 0, STEP_DONE = 1, STEP_OCCLUDED = 2, STEP_OVERFLOW = 3 };
 
 struct TraceScene {
     const float4* __restrict__ nodes;   // binary: 4 float4 per internal node; wide: 8
@@ -230,12 +230,15 @@ MC_D float4 pick(bool c, const float4& a, const float4& b) {
 // and y planes as low low, high high, low high, high low; 8..11 low z and high
 // z, each followed by the references) or MC_BVH_LAYOUT_WIDE4Q (64-byte
 // quantised nodes with conservative boxes: more boxes pass, the leaf tests and
-// the rank rule decide the hit as with exact boxes).
+// the rank rule decide the hit as with exact boxes); with MC_LAYOUT_ORDERED for
+// launches whose stack may be too short.
 template <bool ANY, int ISECT, bool COUNT, class Stack, int FORM>
 MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, const WatertightRay& w, int* err,
                     TravCount* cnt) {
+    constexpr int NODES = FORM & 3;
+    constexpr bool ORDERED = (FORM & MC_LAYOUT_ORDERED) != 0;
     float4 ax, ay, az, bx, by, bz, rf;  // near and far planes of the four children, their references
-    if (FORM == MC_BVH_LAYOUT_WIDE4Q) {
+    if (NODES == MC_BVH_LAYOUT_WIDE4Q) {
         const float4* nd = sc.nodes + (size_t)((unsigned)s.node * 4u);
         float4 h, q0, q1;
         ldg8(nd, h, q0);
@@ -252,7 +255,7 @@ MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, cons
         by = q_planes(h.y, sy, ny ? ly : hy);
         az = q_planes(h.z, sz, nz ? hz : lz);
         bz = q_planes(h.z, sz, nz ? lz : hz);
-    } else if (FORM == MC_BVH_LAYOUT_WIDE4) {
+    } else if (NODES == MC_BVH_LAYOUT_WIDE4) {
         const float4* nd = sc.nodes + (size_t)((unsigned)s.node * 8u);
         float4 lx, ly, lz, hx, hy, hz;
         ldg8(nd, lx, ly);
@@ -289,7 +292,7 @@ MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, cons
     if (COUNT) cnt->visits++;
     unsigned lm = (hit[0] && ref[0] < 0 ? 1u : 0u) | (hit[1] && ref[1] < 0 ? 2u : 0u) |
                   (hit[2] && ref[2] < 0 ? 4u : 0u) | (hit[3] && ref[3] < 0 ? 8u : 0u);
-    // internal children, the nearest first; misses, leaves and empty slots
+    // internal children by distance; misses, leaves and empty slots
     // (MC_WIDE_EMPTY, the largest int) as +inf
     constexpr unsigned kLeafOrEmpty = (unsigned)MC_WIDE_EMPTY;
     float k0 = (hit[0] && (unsigned)ref[0] < kLeafOrEmpty) ? tn[0] : INFINITY;
@@ -300,6 +303,14 @@ MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, cons
     cswap(k0, v0, k1, v1);
     cswap(k2, v2, k3, v3);
     cswap(k0, v0, k2, v2);
+    // The ones to push stay in part order where the stack holds all that a ray of
+    // the tree can push: the full sort costs 6 % of 1M scattered rays. In a shorter
+    // stack (stack_entries) the order decides how many entries a ray needs, and
+    // the farthest goes first.
+    if (ORDERED) {
+        cswap(k1, v1, k3, v3);
+        cswap(k1, v1, k2, v2);
+    }
     int step = STEP_CONTINUE;
     if (k0 == INFINITY) {
         if (s.sp == stack.bottom) step = STEP_DONE;
@@ -311,12 +322,14 @@ MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, cons
         // push the others, continue with the nearest
         const int extra = (k1 != INFINITY) + (k2 != INFINITY) + (k3 != INFINITY);
         if (s.sp + extra * Stack::kStep > stack.limit) {
-            atomicOr(err, MC_DEVERR_STACK);
-            step = STEP_DONE;
+            // ordered: reported after the leaves, one of which may end an occlusion ray
+            if (!ORDERED) atomicOr(err, MC_DEVERR_STACK);
+            step = ORDERED ? STEP_OVERFLOW : STEP_DONE;
         } else {
             if (k3 != INFINITY) { stack.put(s.sp, v3); s.sp += Stack::kStep; }
+            if (ORDERED && k2 != INFINITY) { stack.put(s.sp, v2); s.sp += Stack::kStep; }
             if (k1 != INFINITY) { stack.put(s.sp, v1); s.sp += Stack::kStep; }
-            if (k2 != INFINITY) { stack.put(s.sp, v2); s.sp += Stack::kStep; }
+            if (!ORDERED && k2 != INFINITY) { stack.put(s.sp, v2); s.sp += Stack::kStep; }
             s.node = v0;
         }
     }
@@ -338,10 +351,14 @@ MC_D int trav_step4(const TraceScene& sc, TravState& s, const Stack& stack, cons
             }
         }
     }
+    if (ORDERED && step == STEP_OVERFLOW) {
+        atomicOr(err, MC_DEVERR_STACK);
+        step = STEP_DONE;
+    }
     return step;
 }
 
-// LAY: MC_BVH_LAYOUT_BINARY, _WIDE4, _WIDE4Q or MC_LAYOUT_OCTANT.
+// LAY: MC_BVH_LAYOUT_BINARY, or a FORM of trav_step4.
 template <bool ANY, int ISECT, bool COUNT, int LAY, class Stack>
 MC_D int trav_step_layout(const TraceScene& sc, TravState& s, const Stack& stack, const WatertightRay& w, int* err,
                           TravCount* cnt) {
