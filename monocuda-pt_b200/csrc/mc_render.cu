@@ -337,8 +337,17 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? MC_TRACE_MIN_BLOCKS 
     while (true) {
         const unsigned running = __ballot_sync(kFull, state == LANE_RUNNING);
         // finished rays wait until enough lanes are idle, then one pass writes
-        // all their results and the freed lanes take new rays
-        if (exhausted ? running != kFull : __popc(running) <= floor) {
+        // all their results and the freed lanes take new rays. Once no rays are
+        // left to take, they wait for the warp's last one, but for shadow rays
+        // through media, which may go on behind the boundary they found. (A pass
+        // in every step with a finished lane made the tail of a launch 5 to 15 %
+        // longer: plain closest hits of 1M rays on 20k triangles with the binary
+        // tree 1.12, now 0.99 of the time with results written at once.)
+        bool pass;
+        if (!exhausted) pass = __popc(running) <= floor;
+        else if (MED == 0) pass = running == 0u;
+        else pass = running == 0u || __any_sync(kFull, state > LANE_RUNNING && kind == RAY_SHADOW_MEDIUM);
+        if (pass) {
             if (state > LANE_RUNNING) {
                 const mc_triangle_cold* cold = a.cold0;
                 const mc_sphere* spheres = a.spheres0;
