@@ -1256,19 +1256,54 @@ __global__ void __launch_bounds__(256) k_ratio_track(ShadeArgs a, RatioArgs v) {
 // is, and here a path waits for its own rays only: a 64x48 preview 278 -> 164 us
 // (161 with octant nodes),
 // the 333x180 cloud frame of depth 1000 39.1 -> 11.0 ms (8.8 with the trackers'
-// random numbers drawn ahead). Launched where
-// kPathsInFlight says.
+// random numbers drawn ahead). Launched where whole_wave_limit and hand_over_limit
+// say.
 // Lanes per warp as in k_trace: one path per warp when there are few. What the
 // wave passes through memory (a shadow ray's contribution and length) is rounded
 // there, so its uses here are written with explicit roundings.
+
+// Both limits go by the bounces that may remain: the more of them, the more
+// launches, each as long as its slowest ray, one launch saves. us, the wave's
+// launches / one launch (256x256 x 1, 181x181 and 128x128, 30k-triangle member
+// scene, Cornell spheres, aperture room):
+//   max_depth     65,536 paths                      32,761                            16,384
+//    1            266 / 327, 117 / 127, 246 / 247   242 / 247, 105 / 92,  216 / 211   219 / 197, 97 / 87,   196 / 186
+//    4            618 / 754, 298 / 438, 617 / 976   532 / 592, 263 / 349, 556 / 582   482 / 445, 238 / 264, 524 / 436
+//    8            782 / 855, 445 / 565, 900 / 1224  678 / 658, 405 / 433, 814 / 717   584 / 506, 370 / 346, 753 / 507
+//   20            884 / 884, 671 / 582, 1189 / 1233 764 / 658, 607 / 432, 1054 / 721  671 / 493, 550 / 359, 964 / 522
+// Steps in the binary layout are cheaper and more, and one launch wins up to 64K
+// paths at any depth (room, depth 4: 1361 / 1281, depth 8: 2022 / 1629). With
+// density grids a bounce waits on long chains of voxel reads, every path on its
+// own (cloud, 1,048,576 paths: depth 4 452 / 703, 8 723 / 1073, 20 1405 / 1371,
+// 100 1859 / 1431; 524,176: 338 / 402, 587 / 592, 1261 / 878; 262,144: 277 / 253,
+// 528 / 410, 1157 / 636).
+__host__ __device__ inline int whole_wave_limit(int bounces, bool grid, bool binary) {
+    const int r = bounces < 64 ? bounces : 64;
+    if (grid) return r << 15 < 1 << 17 ? 1 << 17 : r << 15 > 1 << 20 ? 1 << 20 : r << 15;
+    if (binary) return 1 << 16;
+    return r << 12 < 1 << 14 ? 1 << 14 : r << 12 > 1 << 16 ? 1 << 16 : r << 12;
+}
+// Larger waves leave a bounce of few paths, and all after it, to k_paths. Their
+// own launches for those bounces are enqueued all the same, with nothing to do,
+// so there has to be more to gain (hand-over at 16,384 paths whatever the rest,
+// spheres of 128x128: depth 2 149 -> 174 us, depth 4 238 -> 311; at this limit
+// 600x600 spheres of depth 20 take 2.81 -> 2.55 ms, with octant nodes; 1.2M
+// paths of the cloud, depth 8, 710 us without, 890 handed over at 229K).
+__host__ __device__ inline int hand_over_limit(int bounces, bool grid) {
+    const int r = bounces < 32 ? bounces : 32;
+    if (grid) return r << 13;
+    return r < 2 ? 0 : r < 8 ? r << 11 : 1 << 14;
+}
+
 struct PathsArgs {
     // The bounce taken over is the first of depthLo .. depthHi - 1 whose queue
-    // holds between one and `few` paths (the wave's launches left that bounce
-    // alone, so the later queues are empty).
+    // holds between one and `few` paths, or hand_over_limit's of the bounces up
+    // to depthEnd when few is 0 (the wave's launches left that bounce alone, so
+    // the later queues are empty).
     const int* queue[2];
     int* counters;       // of bounce d: slot d, or d % kRingSlots in a deep wave
     int ring;
-    int depthLo, depthHi, few;
+    int depthLo, depthHi, depthEnd, few;
     int stackCap;
     int gridMedia;       // the wave's trace launches would be the density-grid variant
     long long* stats;    // extend and shadow rays per depth
@@ -1360,7 +1395,7 @@ __global__ void __launch_bounds__(kPathsThreads) k_paths(ShadeArgs a, PathsArgs 
     for (int d0 = v.depthLo; d0 < v.depthHi && first < 0; d0 += 32) {
         const int d = d0 + lane;
         const int c = d < v.depthHi ? v.counters[(v.ring ? d % v.ring : d) * MC_COUNTERS_PER_DEPTH] : 0;
-        const unsigned m = __ballot_sync(kFull, c > 0 && c <= v.few);
+        const unsigned m = __ballot_sync(kFull, c > 0 && c <= (v.few ? v.few : hand_over_limit(v.depthEnd - d, v.gridMedia != 0)));
         if (m) first = d0 + __ffs(m) - 1;
     }
     if (first < 0) return;
@@ -1711,22 +1746,6 @@ static void set_single_scene(TraceArgs& t, const mc_bvh* bvh, int root, const mc
     t.spheres0 = v->spheres;
 }
 
-// Waves of at most this many paths run as one k_paths launch, and deep waves
-// (max_depth > MC_MAX_DEPTH_STATS) hand their paths over once so few go on.
-// Where the line lies (paths: wave launches / one launch, us): Cornell boxes
-// 4,096: 298 / 189, 65,536: 372 / 355, 131,044: 436 / 479; spheres, depth 20,
-// 4,096: 472 / 243, 65,536: 726 / 684, 131,044: 857 / 985; icospheres (246k
-// triangles) 883 / 817 and 1043 / 1037. With density grids a bounce waits on
-// long chains of voxel reads and every path on its own: 131,044 paths of the
-// cloud 65,800 / 15,100, 960k 26,100 (handed over at 65,536) / 20,700.
-constexpr int kPathsInFlight = 1 << 16;
-constexpr int kPathsInFlightGrid = 1 << 20;
-// Larger waves leave a bounce with at most this many paths, and all after it,
-// to k_paths (4K to 32K measured alike, 64K slower where the paths are long):
-// 600x600 spheres of depth 20 2.81 -> 2.66 ms (2.55 with octant nodes), 131,044
-// paths 939 -> 739 us, Cornell boxes 493 -> 423 us, 16 small scenes 2.16 -> 2.12 ms.
-constexpr int kHandOver = 1 << 14;
-
 static void launch_paths(mc_context* ctx, cudaStream_t stream, const ShadeArgs& a, PathsArgs v, int form) {
     typedef void (*Kernel)(ShadeArgs, PathsArgs);
     static const Kernel table[8] = {k_paths<0>, k_paths<1>, k_paths<2>, k_paths<3>,
@@ -1944,15 +1963,14 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
     // limit, the plain mode, the reference's per-pixel generators)
     const bool pathsOk = philox && !timeTrace && !countVisits && !alias && isect == MC_ISECT_REFERENCE && persistent &&
                          p0.queue_capacity == 0 && maxD > 0;
-    const int fewPaths = grid ? kPathsInFlightGrid : kPathsInFlight;
-    const int handPaths = grid ? kPathsInFlightGrid : kHandOver;
-    const bool smallWave = pathsOk && !guide && capacity <= fewPaths;
+    const bool binary = bvh->layout == MC_BVH_LAYOUT_BINARY;
+    const bool smallWave = pathsOk && !guide && capacity <= whole_wave_limit(maxD, grid, binary);
     // the first bounce k_paths may take over: guided bounces shade with the
     // guide, and a guided wave's second trace keeps the primary vertices'
     // next-event estimates apart (a deep wave hands over at its read-backs, from
     // the same bounce on)
     const int handFrom = !guide ? 1 : guidedDepth > 0 ? std::max(guidedDepth, 2) : maxD;
-    const bool handOver = pathsOk && !deep && !smallWave && handFrom < maxD;
+    const bool handOver = pathsOk && !deep && !smallWave && hand_over_limit(maxD - handFrom, grid) > 0;
     auto enqueue_paths = [&](int lo, int hi, int few) {
         PathsArgs v;
         std::memset(&v, 0, sizeof(v));
@@ -1962,6 +1980,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
         v.ring = deep ? kRingSlots : 0;
         v.depthLo = lo;
         v.depthHi = hi;
+        v.depthEnd = maxD;
         v.few = few;
         v.stackCap = ta.stackCap;
         v.gridMedia = grid ? 1 : 0;
@@ -2001,7 +2020,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
             if (d > 0) t.shCount = slot(d - 1) + 1;
             else { t.shCount = nullptr; t.shN = 0; }
             t.work = slot(d) + 2;
-            const int leave = handOver && d >= handFrom ? handPaths : 0;  // queues up to this size are left to k_paths
+            const int leave = handOver && d >= handFrom ? hand_over_limit(maxD - d, grid) : 0;  // queues up to this size are left to k_paths
             t.handOver = leave;
             if (guide && d == 1) {
                 // the primary vertex's NEE lands apart from the sample so that
@@ -2026,7 +2045,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
                     enqueue_paths(d, d + 1, capacity);
                     dEnd = d + 1;
                 }
-                if (handOver) enqueue_paths(handFrom, maxD, handPaths);
+                if (handOver) enqueue_paths(handFrom, maxD, 0);
                 break;
             }
             // bounces past the guided depth shade with the cosine lobe alone: no inference
@@ -2085,7 +2104,7 @@ mc_status run_waves(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items, i
                 int next = 0;
                 MC_CUDA(cudaMemcpyAsync(&next, slot(d + 1), sizeof(int), cudaMemcpyDeviceToHost, stream));
                 MC_CUDA(cudaStreamSynchronize(stream));
-                few = pathsOk && d + 1 >= handFrom && next > 0 && next <= fewPaths;
+                few = pathsOk && d + 1 >= handFrom && next > 0 && next <= whole_wave_limit(maxD - (d + 1), grid, binary);
                 stop = next == 0 || few;
             }
         }
