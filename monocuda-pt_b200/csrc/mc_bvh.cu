@@ -2077,7 +2077,6 @@ static mc_status build_wide(mc_context* ctx, mc_bvh* bvh, const Seg* dSeg, int n
         MC_CUDA(cudaMemcpyAsync(bvh->wide_nodes, h, sizeof(h), cudaMemcpyHostToDevice, ctx->stream));
     }
     if ((st = leaf_records(ctx, bvh->prims, rank, N, bvh->records)) != MC_OK) return st;
-    MC_CUDA(cudaStreamSynchronize(ctx->stream));
     bvh->wide_count = count;
     bvh->layout = MC_BVH_LAYOUT_WIDE4;
     return MC_OK;
@@ -2264,6 +2263,8 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
         return s != MC_OK ? s : f ? status_from_device_flags(f) : MC_OK;
     };
     if ((st = leaves(!clusteredOnly)) != MC_OK) return fail(st);
+    // what the binary layout's traversal reads, before the wait for the root boxes
+    if (!wide && (st = leaf_records(ctx, bvh->prims, nullptr, N, bvh->records)) != MC_OK) return fail(st);
     if (!clusteredOnly && (st = root_boxes()) != MC_OK) return fail(st);
     bvh->seg_prim_off.resize(nseg);
     bvh->bin_roots.resize(nseg);
@@ -2312,10 +2313,6 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
         }
         k_quantize_wide<<<grid_for((int)bvh->wide_count, kBlock), kBlock, 0, ctx->stream>>>(
             (const float4*)bvh->wide_nodes, (int)bvh->wide_count, (float4*)q);
-        if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
-            pool_free(ctx, q);
-            return fail(cuda_error(cudaGetLastError(), "mc_bvh_build (quantise)", __FILE__, __LINE__));
-        }
         pool_free(ctx, bvh->wide_nodes);
         bvh->wide_nodes = q;
         bvh->layout = MC_BVH_LAYOUT_WIDE4Q;
@@ -2324,22 +2321,18 @@ mc_status build_segments(mc_context* ctx, const mc_scene_view* views, int nseg, 
         if (palloc(ctx, &bvh->octant_nodes, (size_t)bvh->wide_count * 192)) {
             k_expand_wide<<<grid_for((int)bvh->wide_count, kBlock), kBlock, 0, ctx->stream>>>(
                 (const float4*)bvh->wide_nodes, (int)bvh->wide_count, (float4*)bvh->octant_nodes);
-            if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-                return fail(cuda_error(cudaGetLastError(), "mc_bvh_build (octant nodes)", __FILE__, __LINE__));
         } else {
             cudaGetLastError();  // no room: traversal reads the 128-byte nodes
             bvh->octant_nodes = nullptr;
         }
     }
-    if (bvh->layout == MC_BVH_LAYOUT_BINARY) {
-        if ((st = leaf_records(ctx, bvh->prims, nullptr, N, bvh->records)) != MC_OK) return fail(st);
-        if (cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-            return fail(cuda_error(cudaGetLastError(), "mc_bvh_build (leaf records)", __FILE__, __LINE__));
-    }
     if (wide) {
         bvh->device_bytes += bvh->wide_count * (bvh->layout == MC_BVH_LAYOUT_WIDE4Q ? 64 : 128) +
                              (bvh->octant_nodes ? bvh->wide_count * 192 : 0);
         bvh->nodes = nullptr;  // the build's: traversal reads the wide nodes
+        // the collapse's last copies and kernels
+        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+            return fail(cuda_error(cudaGetLastError(), "mc_bvh_build (wide nodes)", __FILE__, __LINE__));
     }
     pool_free(ctx, bvh->work);
     bvh->work = bvh->prims = nullptr;
