@@ -219,12 +219,14 @@ MC_D bool hit_sphere_ref(const V3& c0, const V3& c1, bool moving, float radius, 
                          float& tout, bool& frontFace, V3& outward) {
     V3 cc = sphere_center_at(c0, c1, moving, time);
     V3 oc = cc - o;
-    // |d|^2 with its contraction written out: left to the compiler, which of
-    // the first two squares is rounded depends on the code around the call
-    float dd = __fmaf_rn(d.z, d.z, __fmaf_rn(d.x, d.x, __fmul_rn(d.y, d.y)));
-    float tc = oc.dot(d) / dd;
+    // The dot products with their contraction written out: left to the compiler,
+    // which of the first two products is rounded depends on the code around the
+    // call, and the same ray would hit the same sphere elsewhere in another kernel
+    auto dot = [](const V3& u, const V3& v) { return __fmaf_rn(u.z, v.z, __fmaf_rn(u.x, v.x, __fmul_rn(u.y, v.y))); };
+    float tc = dot(oc, d) / dot(d, d);
     V3 closest = o + d * tc;
-    float dist2 = (cc - closest).length_squared();
+    V3 off = cc - closest;
+    float dist2 = dot(off, off);
     float disc = radius * radius - dist2;
     if (disc < 0.0f) return false;
     float half = sqrtf(disc);

@@ -578,15 +578,17 @@ MC_D void train_remainder(const ShadeArgs& a, int p, int depth, const V3& L, flo
 // Dot product with its contraction written out: left to the compiler, which of
 // the first two products is rounded follows how often each is used in the code
 // around the call, so the same shading would round differently in k_shade and
-// k_paths. These are the choices it made for k_shade, whose XORWOW instance
-// differs from the Philox one in the diffuse density only.
+// k_paths. These are the choices it made for k_shade: every product of a next
+// event's directions as in shade_dot; the cosines of the emission weight and of
+// the sampled direction's density (bsdf_dot) as there for Philox, the other way
+// for XORWOW.
 MC_D float shade_dot(const V3& u, const V3& v) { return __fmaf_rn(u.z, v.z, __fmaf_rn(u.y, v.y, __fmul_rn(u.x, v.x))); }
 template <class Rng>
-MC_D float diffuse_dot(const V3& u, const V3& v) {
+MC_D float bsdf_dot(const V3& u, const V3& v) {
     return shade_dot(u, v);
 }
 template <>
-MC_D float diffuse_dot<XorwowRng>(const V3& u, const V3& v) {
+MC_D float bsdf_dot<XorwowRng>(const V3& u, const V3& v) {
     return __fmaf_rn(u.z, v.z, __fmaf_rn(u.x, v.x, __fmul_rn(u.y, v.y)));
 }
 
@@ -664,7 +666,7 @@ MC_D void shade_path(const ShadeArgs& a, const SceneGPU& S, int p, int depth, Sh
         float emissionWeight = 1.0f;
         bool fromBsdf = !(depth == 0 || prevSpec);
         if (fromBsdf && ptype == 1) {
-            float cosL = fmaxf(fabsf(shade_dot(inDir, hitNormal)), 1e-4f);
+            float cosL = fmaxf(fabsf(bsdf_dot<Rng>(inDir, hitNormal)), 1e-4f);
             float area = triangle_area(tv0, tv1, tv2);
             float lightPdf = light_solid_angle_pdf((1.0f - env_selection_probability(S.env, lightCount)) / float(lightCount),
                                                    hitT, cosL, area);
@@ -826,9 +828,9 @@ MC_D void shade_path(const ShadeArgs& a, const SceneGPU& S, int p, int depth, Sh
         a.tg[p] = throughput.y;
         a.tb[p] = throughput.z;
         a.spec[p] = (mat.type != MC_MAT_LAMBERTIAN && mat.type != MC_MAT_ISOTROPIC) ? 1 : 0;
-        a.pdf[p] = (mat.type == MC_MAT_ISOTROPIC) ? hg_phase_pdf(shade_dot(inDir, nd), mat.g)
+        a.pdf[p] = (mat.type == MC_MAT_ISOTROPIC) ? hg_phase_pdf(bsdf_dot<Rng>(inDir, nd), mat.g)
                    : (GUIDED && mat.type == MC_MAT_LAMBERTIAN) ? guidedPdf
-                                                               : lambertian_cosine_pdf(fmaxf(diffuse_dot<Rng>(nd, hitNormal), 0.0f));
+                                                               : lambertian_cosine_pdf(fmaxf(bsdf_dot<Rng>(nd, hitNormal), 0.0f));
         out.next = depth + 1 < S.maxDepth;  // the scene's max depth ends the path (PT:3793)
     }
     rng_store<Rng>(a, S, p, rng);
