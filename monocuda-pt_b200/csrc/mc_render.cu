@@ -2325,6 +2325,15 @@ mc_status render_items(mc_context* ctx, const mc_bvh* bvh, const WaveItem* items
     return finish_stats(ctx, tm, paths, stats);
 }
 
+// Closest-hit sets of at most this many rays push in full order: such a launch
+// lasts as long as its longest ray, and part order lengthens some rays by a third.
+// Against results in the order of before the part sort, 1,000 and 5,003 rays on
+// seven scenes, persistent and plain, reference intersector: part order 0.89 to
+// 1.02 (worst scene 1.28), full 0.87 to 0.97 (1.07); 20,000 rays 0.92 to 0.96
+// against 0.95 to 0.97. Occlusion rays end early, and part order is the better one
+// at any number (5,003: 0.89 to 0.97 against 0.91 to 0.98).
+constexpr int kOrderedRays = 1 << 13;
+
 // The single-scene trace arguments and launch shape of the ray-set entry points.
 static void ray_set_scene(TraceArgs& t, const mc_bvh* bvh, const mc_scene_view* scene, int isect) {
     default_shape(t, shape_levels(bvh), isect);
@@ -2475,7 +2484,8 @@ mc_status mc_trace_closest(mc_context* ctx, const mc_bvh* bvh, const mc_scene_vi
     t.dx = d_rays + 3 * N; t.dy = d_rays + 4 * N; t.dz = d_rays + 5 * N; t.time = d_rays + 6 * N;
     t.hits = d_hits;
     t.work = work;
-    mc::launch_trace(ctx, ctx->stream, t, mc::traversal_form(bvh), false, intersector, !plain, (n + 255) / 256);
+    const int form = mc::traversal_form(bvh) | (n <= mc::kOrderedRays ? MC_LAYOUT_ORDERED : 0);
+    mc::launch_trace(ctx, ctx->stream, t, form, false, intersector, !plain, (n + 255) / 256);
     MC_CUDA(cudaGetLastError());
     int flags = 0;
     MC_CUDA(cudaMemcpyAsync(&flags, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));

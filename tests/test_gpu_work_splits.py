@@ -1,7 +1,8 @@
 """The sizes at which kernels split their work differently. Clustering: tiles of
 240 positions, one block alone up to four tiles (960). Persistent traversal: a
 warp takes as many lanes as its share of the rays, 1 to 32, with 32 resident
-warps per SM (4-wide trees, 128-thread blocks) or 24 (256-thread blocks)."""
+warps per SM (4-wide trees, 128-thread blocks) or 24 (256-thread blocks); sets of
+at most 8,192 closest-hit rays push children in full order."""
 import ctypes as C
 
 import numpy as np
@@ -56,7 +57,7 @@ def counts(per_sm):
     out = []
     for k in (1, 2, 3, 8, 17, 30, 31, 32):
         out += [k * warps - 1, k * warps, k * warps + 1]
-    return out + [33 * warps + 5]
+    return out + [33 * warps + 5, 8191, 8192, 8193]  # closest hits push in full order up to 8192
 
 
 @pytest.mark.parametrize("layout,per_sm", [(mcpt.LAYOUT_WIDE4, 32), (mcpt.LAYOUT_WIDE4Q, 32), (mcpt.LAYOUT_BINARY, 24)])
